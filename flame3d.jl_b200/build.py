@@ -31,6 +31,9 @@ PER_FILE = {
     "kernels_ref.cu": ["-fmad=false"],
     "chemistry.cu": ["-fmad=false"],
 }
+# Compiled once per species count (the object files compile side by side).
+PER_SPECIES = {"pencil_inst.cu": ("FLAME_PENCIL_NS", range(1, 10)),
+               "fused_inst.cu": ("FLAME_FUSED_NS", range(1, 10))}
 
 
 def nvcc() -> str:
@@ -61,9 +64,22 @@ def needs_build() -> bool:
     return any(p.stat().st_mtime > t for p in sources() + headers() + [Path(__file__)])
 
 
-def compile_one(src: Path, verbose_ptxas: bool) -> Path:
-    obj = BUILD / (src.stem + ".o")
-    cmd = [nvcc(), *host_compiler(), *ARCH, *COMMON, *PER_FILE.get(src.name, []), "-c",
+def units() -> list[tuple[Path, str, list[str]]]:
+    """(source, object name, extra flags) of every object file, the longest to compile first."""
+    out = []
+    for src in sources():
+        macro, values = PER_SPECIES.get(src.name, (None, None))
+        if macro:
+            out += [(src, f"{src.stem}_{v}.o", [f"-D{macro}={v}"]) for v in values]
+        else:
+            out.append((src, src.stem + ".o", []))
+    return sorted(out, key=lambda u: u[1], reverse=True)
+
+
+def compile_one(unit: tuple[Path, str, list[str]], verbose_ptxas: bool) -> Path:
+    src, name, flags = unit
+    obj = BUILD / name
+    cmd = [nvcc(), *host_compiler(), *ARCH, *COMMON, *PER_FILE.get(src.name, []), *flags, "-c",
            str(src), "-o", str(obj)]
     if verbose_ptxas:
         cmd += ["-Xptxas", "-v"]
@@ -98,7 +114,7 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
         return LIB
     BUILD.mkdir(exist_ok=True)
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        objs = list(ex.map(lambda s: compile_one(s, verbose_ptxas), sources()))
+        objs = list(ex.map(lambda u: compile_one(u, verbose_ptxas), units()))
     tmp = LIB.with_suffix(".so.tmp")
     cmd = [nvcc(), *host_compiler(), *ARCH, "-shared", "-o", str(tmp), *map(str, objs)]
     r = subprocess.run(cmd, capture_output=True, text=True)

@@ -237,7 +237,7 @@ __device__ __forceinline__ T minmod(T a, T b) {  // schemes.jl:26-28
 // WENO-Z weights and combination, schemes.jl:152-162, for the 1:1 kernels: the smoothness
 // indicators come in the arithmetic type T and the weights are formed in FP64 in the reference's
 // four-division form (in plain FP32, q = τ/(1e-26 + β) overflows when a one-sided split makes β
-// exactly 0, and ∞·0 would poison the flux; wenoz_combine_fast<float> below avoids that).
+// exactly 0, and ∞·0 would poison the flux; wenoz_combine_fast below avoids that).
 template <typename T>
 __device__ __forceinline__ T wenoz_combine(T s11_, T s22_, T s33_, T v1, T v2, T v3) {
     const double s11 = s11_, s22 = s22_, s33 = s33_;
@@ -280,32 +280,76 @@ __device__ __forceinline__ T wenoz_minus(T V1, T V2, T V3, T V4, T V5) {
                             2 * V3 + 5 * V2 - V1);
 }
 
-// The same WENO-Z combination with one division instead of four: with b_k = ε + β_k,
-// α_k = d_k (1 + τ²/b_k²) and ω_k = α_k / Σα; multiplying every α_k by b_1² b_2² b_3² gives
-// A_k = d_k (b_k² + τ²) Π_{j≠k} b_j² with the same ratios.  Exact in real arithmetic; in FP64 it
-// differs from the reference's rounding by a few ulp (the products stay in range for |β| < 1e50).
-template <typename T>
-__device__ __forceinline__ T wenoz_combine_fast(T s11_, T s22_, T s33_, T v1, T v2, T v3) {
-    const double b1 = kWenoEps + double(s11_), b2 = kWenoEps + double(s22_),
-                 b3 = kWenoEps + double(s33_);
-    const double tau = fabs(double(s11_) - double(s33_));
-    const double t = tau * tau;
-    const double p1 = b1 * b1, p2 = b2 * b2, p3 = b3 * b3;
-    const double a1 = (p1 + t) * (p2 * p3);
-    const double a2 = 6.0 * (p2 + t) * (p1 * p3);
-    const double a3 = 3.0 * (p3 + t) * (p1 * p2);
-    return T((a1 * double(v1) + a2 * double(v2) + a3 * double(v3)) / (6.0 * (a1 + a2 + a3)));
+// Reciprocal and reciprocal square root for the fused FP64 paths: the hardware's approximation
+// (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64) refined by Newton's iteration, without the
+// branches of the correctly rounded forms.  The seed is good to about 2^-20 and one step of third
+// order, x (1 + e + e^2) with e = 1 - d x, leaves it below 2^-57 before the rounding of the last
+// multiply-add.  Arguments are normal, positive or negative (rsqrt: positive); other arguments
+// give NaN or infinity.
+__device__ __forceinline__ double fast_rcp(double d) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    const double e = fma(-d, x, 1.0);
+    return fma(x, fma(e, e, e), x);
+}
+// x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2
+__device__ __forceinline__ double fast_rsqrt(double d) {
+    double x;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    const double e = fma(-d * x, x, 1.0);
+    return fma(x * e, fma(0.375, e, 0.5), x);
 }
 
-// FP32 form for the mixed-precision paths, in the reference's own shape α_k = d_k (1 + q_k²),
+// max that propagates NaN (Julia's) in the arithmetic type
+template <typename T>
+__device__ __forceinline__ T nmax(T a, T b) {
+    return (a > b || a != a) ? a : b;
+}
+
+// WENO-Z5 of the fused FP64 paths, schemes.jl:139-187, for a stencil V1..V5 in upwind order (the
+// negative flux passes its points reversed), written with the first differences e_k = V_{k+1} -
+// V_k and the second differences a_k = e_{k+1} - e_k:
+//   4 β_k = (13/3) a_k^2 + b_k^2,  b = a_1 + 2 e_2,  e_2 + e_3,  a_3 - 2 e_3
+//   6 v_k = 6 V3 + r_k,            r = 5 e_2 - 2 e_1,  e_2 + 2 e_3,  4 e_3 - e_4
+// so the face value is V3 + (1/6) Σ α_k r_k / Σ α_k, with the reference's weights
+// α_k = d_k (1 + q_k^2), q_k = τ / (ε + β_k), d = 1, 6, 3 (the factor 4 cancels in q).  The
+// same value in real arithmetic, with a third fewer operations than from the V_k, and the
+// rounding of the weighted part only touches the correction to V3.  The sweeps are bound by FP64
+// issue and latency: this, fast_rcp and the split below took an FP64 step of the 256x128x128 jet
+// from 6.75 to 6.34 ms, 101x75x63 with five species from 2.00 to 1.80 ms, 32^3 from 139 to 129 us.
+//
+// Σ α_k r_k / Σ α_k comes as a fraction N / D without divisions: multiplying every α_k by
+// b_1^2 b_2^2 b_3^2 gives A_k = d_k (b_k^2 + τ^2) Π_{j≠k} b_j^2 with the same ratios (the
+// products stay in range for |β| < 1e49).
+__device__ __forceinline__ void weno_fraction(double V1, double V2, double V3, double V4,
+                                              double V5, double &N, double &D) {
+    const double e1 = V2 - V1, e2 = V3 - V2, e3 = V4 - V3, e4 = V5 - V4;
+    const double s1 = e2 - e1, s2 = e3 - e2, s3 = e4 - e3;
+    const double c1 = s1 + 2 * e2, c2 = e2 + e3, c3 = s3 - 2 * e3;
+    const double k = 13.0 / 3.0, eps = 4 * kWenoEps;
+    const double b1 = fma(k * s1, s1, fma(c1, c1, eps));  // 4 (ε + β_k)
+    const double b2 = fma(k * s2, s2, fma(c2, c2, eps));
+    const double b3 = fma(k * s3, s3, fma(c3, c3, eps));
+    const double m = 12 * e3;  // the candidates' corrections: r_1, 6 r_2, 3 r_3 (d_k folded in)
+    const double r1 = fma(5.0, e2, -2 * e1), r2 = fma(6.0, e2, m), r3 = fma(-3.0, e4, m);
+    const double tau = b1 - b3;
+    const double p1 = b1 * b1, p2 = b2 * b2, p3 = b3 * b3;
+    const double a1 = fma(tau, tau, p1) * (p2 * p3);
+    const double a2 = fma(tau, tau, p2) * (p1 * p3);
+    const double a3 = fma(tau, tau, p3) * (p1 * p2);
+    N = fma(a1, r1, fma(a2, r2, a3 * r3));
+    D = fma(6.0, a2, fma(3.0, a3, a1));
+}
+
+// FP32 (the mixed-precision paths), from the V_k: the rounding of the mixed path decides faces whose
+// sensor lies at a branch threshold, so its operations are left as they are.  In the reference's own shape α_k = d_k (1 + q_k²),
 // q_k = τ / (ε + β_k), with every step kept inside FP32 range: q_k is capped at 1e15 (a stencil
 // with q_k that large already carries weight 1 to FP32 precision; when two are capped their
 // candidate values agree to far below FP32 resolution, since β_k < 1e-15 τ bounds their second
 // differences), the α_k are normalised by their sum before they multiply the candidates, and
 // the divisions are the fast approximate ones (2 ulp), ample for weights in FP32.
-template <>
-__device__ __forceinline__ float wenoz_combine_fast<float>(float s11, float s22, float s33,
-                                                           float v1, float v2, float v3) {
+__device__ __forceinline__ float wenoz_combine_fast(float s11, float s22, float s33, float v1,
+                                                    float v2, float v3) {
     constexpr float eps = float(kWenoEps), qmax = 1e15f;
     const float tau = fabsf(s11 - s33);
     const float q1 = fminf(__fdividef(tau, eps + s11), qmax);
@@ -316,78 +360,34 @@ __device__ __forceinline__ float wenoz_combine_fast<float>(float s11, float s22,
     return (1.0f / 6.0f) * ((a1 * r) * v1 + (a2 * r) * v2 + (a3 * r) * v3);
 }
 
-// wenoz_combine_fast<double> as a fraction N / D (so two faces can share one division).
-__device__ __forceinline__ void wenoz_fraction(double s11, double s22, double s33, double v1,
-                                               double v2, double v3, double &N, double &D) {
-    const double b1 = kWenoEps + s11, b2 = kWenoEps + s22, b3 = kWenoEps + s33;
-    const double tau = fabs(s11 - s33);
-    const double t = tau * tau;
-    const double p1 = b1 * b1, p2 = b2 * b2, p3 = b3 * b3;
-    const double a1 = (p1 + t) * (p2 * p3);
-    const double a2 = 6.0 * (p2 + t) * (p1 * p3);
-    const double a3 = 3.0 * (p3 + t) * (p1 * p2);
-    N = a1 * v1 + a2 * v2 + a3 * v3;
-    D = 6.0 * (a1 + a2 + a3);
-}
-
-__device__ __forceinline__ void wenoz_plus_fraction(double V1, double V2, double V3, double V4,
-                                                    double V5, double &N, double &D) {
-    const double tmp1 = 13.0 / 12.0, q4 = 0.25;
-    double a, b;
+__device__ __forceinline__ float wenoz_plus_fast(float V1, float V2, float V3, float V4, float V5) {
+    const float tmp1 = float(13.0 / 12.0), q4 = float(0.25);
+    float a, b;
     a = V1 - 2 * V2 + V3, b = V1 - 4 * V2 + 3 * V3;
-    const double s11 = tmp1 * (a * a) + q4 * (b * b);
+    const float s11 = tmp1 * (a * a) + q4 * (b * b);
     a = V2 - 2 * V3 + V4, b = V2 - V4;
-    const double s22 = tmp1 * (a * a) + q4 * (b * b);
+    const float s22 = tmp1 * (a * a) + q4 * (b * b);
     a = V3 - 2 * V4 + V5, b = 3 * V3 - 4 * V4 + V5;
-    const double s33 = tmp1 * (a * a) + q4 * (b * b);
-    wenoz_fraction(s11, s22, s33, 2 * V1 - 7 * V2 + 11 * V3, -V2 + 5 * V3 + 2 * V4,
-                   2 * V3 + 5 * V4 - V5, N, D);
-}
-
-__device__ __forceinline__ void wenoz_minus_fraction(double V1, double V2, double V3, double V4,
-                                                     double V5, double &N, double &D) {
-    const double tmp1 = 13.0 / 12.0, q4 = 0.25;
-    double a, b;
-    a = V5 - 2 * V4 + V3, b = V5 - 4 * V4 + 3 * V3;
-    const double s11 = tmp1 * (a * a) + q4 * (b * b);
-    a = V2 - 2 * V3 + V4, b = V4 - V2;
-    const double s22 = tmp1 * (a * a) + q4 * (b * b);
-    a = V3 - 2 * V2 + V1, b = 3 * V3 - 4 * V2 + V1;
-    const double s33 = tmp1 * (a * a) + q4 * (b * b);
-    wenoz_fraction(s11, s22, s33, 11 * V3 - 7 * V4 + 2 * V5, -V4 + 5 * V3 + 2 * V2,
-                   2 * V3 + 5 * V2 - V1, N, D);
-}
-
-template <typename T>
-__device__ __forceinline__ T wenoz_plus_fast(T V1, T V2, T V3, T V4, T V5) {
-    const T tmp1 = T(13.0 / 12.0), q4 = T(0.25);
-    T a, b;
-    a = V1 - 2 * V2 + V3, b = V1 - 4 * V2 + 3 * V3;
-    const T s11 = tmp1 * (a * a) + q4 * (b * b);
-    a = V2 - 2 * V3 + V4, b = V2 - V4;
-    const T s22 = tmp1 * (a * a) + q4 * (b * b);
-    a = V3 - 2 * V4 + V5, b = 3 * V3 - 4 * V4 + V5;
-    const T s33 = tmp1 * (a * a) + q4 * (b * b);
-    return wenoz_combine_fast<T>(s11, s22, s33, 2 * V1 - 7 * V2 + 11 * V3, -V2 + 5 * V3 + 2 * V4,
+    const float s33 = tmp1 * (a * a) + q4 * (b * b);
+    return wenoz_combine_fast(s11, s22, s33, 2 * V1 - 7 * V2 + 11 * V3, -V2 + 5 * V3 + 2 * V4,
                                  2 * V3 + 5 * V4 - V5);
 }
 
-template <typename T>
-__device__ __forceinline__ T wenoz_minus_fast(T V1, T V2, T V3, T V4, T V5) {
-    const T tmp1 = T(13.0 / 12.0), q4 = T(0.25);
-    T a, b;
+__device__ __forceinline__ float wenoz_minus_fast(float V1, float V2, float V3, float V4, float V5) {
+    const float tmp1 = float(13.0 / 12.0), q4 = float(0.25);
+    float a, b;
     a = V5 - 2 * V4 + V3, b = V5 - 4 * V4 + 3 * V3;
-    const T s11 = tmp1 * (a * a) + q4 * (b * b);
+    const float s11 = tmp1 * (a * a) + q4 * (b * b);
     a = V2 - 2 * V3 + V4, b = V4 - V2;
-    const T s22 = tmp1 * (a * a) + q4 * (b * b);
+    const float s22 = tmp1 * (a * a) + q4 * (b * b);
     a = V3 - 2 * V2 + V1, b = 3 * V3 - 4 * V2 + V1;
-    const T s33 = tmp1 * (a * a) + q4 * (b * b);
-    return wenoz_combine_fast<T>(s11, s22, s33, 11 * V3 - 7 * V4 + 2 * V5, -V4 + 5 * V3 + 2 * V2,
+    const float s33 = tmp1 * (a * a) + q4 * (b * b);
+    return wenoz_combine_fast(s11, s22, s33, 11 * V3 - 7 * V4 + 2 * V5, -V4 + 5 * V3 + 2 * V2,
                                  2 * V3 + 5 * V2 - V1);
 }
 
-// One face of the hybrid scheme for the fused paths: hybrid_face7 (below) with the
-// one-division WENO-Z weights.
+// One face of the hybrid scheme for the fused paths: hybrid_face7 (below) with WENO-Z in
+// difference form.
 template <typename T>
 __device__ __forceinline__ T hybrid_face_fast(const T *p, const T *m, T phif) {
     T fp, fm;
@@ -401,11 +401,15 @@ __device__ __forceinline__ T hybrid_face_fast(const T *p, const T *m, T phif) {
             // FP64: F+ and F- share one division, Np/Dp + Nm/Dm = (Np Dm + Nm Dp) / (Dp Dm),
             // while the product of the denominators stays inside the normal range
             double Np, Dp, Nm, Dm;
-            wenoz_plus_fraction(p[0], p[1], p[2], p[3], p[4], Np, Dp);
-            wenoz_minus_fraction(m[1], m[2], m[3], m[4], m[5], Nm, Dm);
+            weno_fraction(p[0], p[1], p[2], p[3], p[4], Np, Dp);
+            weno_fraction(m[5], m[4], m[3], m[2], m[1], Nm, Dm);
             const double den = Dp * Dm;
-            if (den > 1e-300 && den < 1e300) return (Np * Dm + Nm * Dp) / den;
-            return Np / Dp + Nm / Dm;
+            double corr;
+            if (den > 1e-300 && den < 1e300)
+                corr = fma(Np, Dm, Nm * Dp) * fast_rcp(den);
+            else
+                corr = Np / Dp + Nm / Dm;
+            return fma(1.0 / 6.0, corr, p[2] + m[3]);
         } else {
             fp = wenoz_plus_fast(p[0], p[1], p[2], p[3], p[4]);
             fm = wenoz_minus_fast(m[1], m[2], m[3], m[4], m[5]);
@@ -415,6 +419,89 @@ __device__ __forceinline__ T hybrid_face_fast(const T *p, const T *m, T phif) {
         fm = m[3] - T(0.5) * minmod(m[4] - m[3], m[3] - m[2]);
     }
     return fp + fm;
+}
+
+// Steger-Warming splitting of one point, split.jl:17-89, for the fused paths; returns the
+// contravariant velocity A·u.
+//
+// FP64: with h = p + e (so γ = h / e, γ - 1 = p / e and c² = γ p / ρ) the reference's terms
+// collapse: ρ/(2γ) = ρ e / (2h); the acoustic kinetic terms |u ∓ c n|²/2 = k ∓ c θ + c²/2 with
+// k = |u|²/2 and θ = u·n; and ρ/(2γ) (c²/2 + W2) = e / 2.  Equal in real arithmetic; one
+// reciprocal of e ρ h instead of the divisions, and each half of the split costs fifteen
+// operations.
+__device__ __forceinline__ double split_fast(double rho, double u, double v, double w, double p,
+                                             double ei, double A1, double A2, double A3,
+                                             double *fp, double *fm) {
+    const double hh = p + ei, er = ei * rho;
+    const double inv = fast_rcp(er * hh);
+    const double rh = inv * er, q1 = inv * hh;  // 1 / h and 1 / (e ρ)
+    const double c2 = hh * p * q1;
+    const double cs = c2 * fast_rsqrt(c2);
+    const double r2 = A1 * A1 + A2 * A2 + A3 * A3;
+    const double rs = fast_rsqrt(r2);
+    const double E1 = A1 * u + A2 * v + A3 * w;
+    const double css = cs * (r2 * rs);
+    const double E2 = E1 - css, E3 = E1 + css;
+    const double B1 = A1 * rs, B2 = A2 * rs, B3 = A3 * rs, th = E1 * rs;
+    const double E1P = (E1 + fabs(E1)) * 0.5, E2P = (E2 + fabs(E2)) * 0.5,
+                 E3P = (E3 + fabs(E3)) * 0.5;
+    const double E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
+    const double t1 = 0.5 * er * rh;         // ρ / (2γ)
+    const double g2 = 2 * (p * rho) * q1;    // 2 (γ - 1)
+    const double k = 0.5 * (u * u + v * v + w * w), he = 0.5 * ei;
+    const double tc = t1 * cs;
+    {
+        const double s = E2P + E3P, d = tc * (E3P - E2P), m = t1 * fma(g2, E1P, s);
+        fp[0] = m;
+        fp[1] = fma(d, B1, m * u), fp[2] = fma(d, B2, m * v), fp[3] = fma(d, B3, m * w);
+        fp[4] = fma(d, th, fma(m, k, he * s));
+    }
+    {
+        const double s = E2M + E3M, d = tc * (E3M - E2M), m = t1 * fma(g2, E1M, s);
+        fm[0] = m;
+        fm[1] = fma(d, B1, m * u), fm[2] = fma(d, B2, m * v), fm[3] = fma(d, B3, m * w);
+        fm[4] = fma(d, th, fma(m, k, he * s));
+    }
+    return E1;
+}
+
+// FP32: the reference's form with its divisions folded into two reciprocals and an rsqrt.
+__device__ __forceinline__ float split_fast(float rho, float u, float v, float w, float p,
+                                            float ei, float A1, float A2, float A3, float *fp,
+                                            float *fm) {
+    const float h = 0.5f;
+    const float gam = p * (1.0f / ei) + 1;
+    const float gm1 = gam - 1;
+    const float inv = 1.0f / (rho * gam * gm1);  // 1 / (ρ γ (γ-1))
+    const float cs = sqrt(gam * p * (gam * gm1 * inv));
+    const float r2 = A1 * A1 + A2 * A2 + A3 * A3;
+    const float rs = rsqrt(r2);
+    const float ss = r2 * rs;
+    const float E1 = A1 * u + A2 * v + A3 * w;
+    const float E2 = E1 - cs * ss, E3 = E1 + cs * ss;
+    const float B1 = A1 * rs, B2 = A2 * rs, B3 = A3 * rs;
+    const float E1P = (E1 + fabs(E1)) * h, E2P = (E2 + fabs(E2)) * h, E3P = (E3 + fabs(E3)) * h;
+    const float E1M = E1 - E1P, E2M = E2 - E2P, E3M = E3 - E3P;
+    const float uc1 = u - cs * B1, uc2 = u + cs * B1;
+    const float vc1 = v - cs * B2, vc2 = v + cs * B2;
+    const float wc1 = w - cs * B3, wc2 = w + cs * B3;
+    const float vvc1 = (uc1 * uc1 + vc1 * vc1 + wc1 * wc1) * h;
+    const float vvc2 = (uc2 * uc2 + vc2 * vc2 + wc2 * wc2) * h;
+    const float vv = gm1 * (u * u + v * v + w * w);
+    const float W2 = (3 - gam) * (h * rho * gam * inv) * (cs * cs);  // (3-γ)/(2(γ-1)) c²
+    const float tmp1 = h * rho * (rho * gm1 * inv);                  // ρ/(2γ)
+    const float tmp2 = 2 * gm1;
+    fp[0] = tmp1 * (tmp2 * E1P + E2P + E3P);
+    fp[1] = tmp1 * (tmp2 * E1P * u + E2P * uc1 + E3P * uc2);
+    fp[2] = tmp1 * (tmp2 * E1P * v + E2P * vc1 + E3P * vc2);
+    fp[3] = tmp1 * (tmp2 * E1P * w + E2P * wc1 + E3P * wc2);
+    fp[4] = tmp1 * (E1P * vv + E2P * vvc1 + E3P * vvc2 + W2 * (E2P + E3P));
+    fm[0] = tmp1 * (tmp2 * E1M + E2M + E3M);
+    fm[1] = tmp1 * (tmp2 * E1M * u + E2M * uc1 + E3M * uc2);
+    fm[2] = tmp1 * (tmp2 * E1M * v + E2M * vc1 + E3M * vc2);
+    fm[3] = tmp1 * (tmp2 * E1M * w + E2M * wc1 + E3M * wc2);
+    fm[4] = tmp1 * (E1M * vv + E2M * vvc1 + E3M * vvc2 + W2 * (E2M + E3M));
+    return E1;
 }
 
 // One face of the hybrid scheme, schemes.jl:110-199.  p[0..6] = F+[c-3..c+3] (F+[c-4] has
