@@ -341,6 +341,17 @@ __device__ __forceinline__ void weno_fraction(double V1, double V2, double V3, d
     D = fma(6.0, a2, fma(3.0, a3, a1));
 }
 
+// The corrections of F+ (stencil P1..P5) and F- (M1..M5, reversed) together.  Each denominator is
+// a normal number (at least 10 ε^6 = 1e-155), so no branch guards its reciprocal.
+__device__ __forceinline__ double weno_corrections(double P1, double P2, double P3, double P4,
+                                                   double P5, double M1, double M2, double M3,
+                                                   double M4, double M5) {
+    double Np, Dp, Nm, Dm;
+    weno_fraction(P1, P2, P3, P4, P5, Np, Dp);
+    weno_fraction(M1, M2, M3, M4, M5, Nm, Dm);
+    return 1.0 / 6.0 * fma(Np, fast_rcp(Dp), Nm * fast_rcp(Dm));
+}
+
 // FP32 (the mixed-precision paths), from the V_k: the rounding of the mixed path decides faces whose
 // sensor lies at a branch threshold, so its operations are left as they are.  In the reference's own shape α_k = d_k (1 + q_k²),
 // q_k = τ / (ε + β_k), with every step kept inside FP32 range: q_k is capped at 1e15 (a stencil
@@ -398,18 +409,8 @@ __device__ __forceinline__ T hybrid_face_fast(const T *p, const T *m, T phif) {
              T(kUP7_3) * m[4] + T(kUP7_2) * m[5];
     } else if (phif < T(kHybrid2)) {
         if constexpr (sizeof(T) == 8) {
-            // FP64: F+ and F- share one division, Np/Dp + Nm/Dm = (Np Dm + Nm Dp) / (Dp Dm),
-            // while the product of the denominators stays inside the normal range
-            double Np, Dp, Nm, Dm;
-            weno_fraction(p[0], p[1], p[2], p[3], p[4], Np, Dp);
-            weno_fraction(m[5], m[4], m[3], m[2], m[1], Nm, Dm);
-            const double den = Dp * Dm;
-            double corr;
-            if (den > 1e-300 && den < 1e300)
-                corr = fma(Np, Dm, Nm * Dp) * fast_rcp(den);
-            else
-                corr = Np / Dp + Nm / Dm;
-            return fma(1.0 / 6.0, corr, p[2] + m[3]);
+            return p[2] + m[3] +
+                   weno_corrections(p[0], p[1], p[2], p[3], p[4], m[5], m[4], m[3], m[2], m[1]);
         } else {
             fp = wenoz_plus_fast(p[0], p[1], p[2], p[3], p[4]);
             fm = wenoz_minus_fast(m[1], m[2], m[3], m[4], m[5]);

@@ -12,7 +12,7 @@ template <>
 const PencilOps &pencil_ops<FLAME_PENCIL_NS>() {
     constexpr int N = FLAME_PENCIL_NS;
     static const PencilOps ops = {
-        {launch<N, double, double>, launch<N, float, float>},
+        {launch<N, double>, launch<N, float>},
         {batch_dims<N, double, double>, batch_dims<N, float, float>},
         {batch_grid<N, double, double>, batch_grid<N, float, float>},
         {batch_launch<N, double, double>, batch_launch<N, float, float>}};

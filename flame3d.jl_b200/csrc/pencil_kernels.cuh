@@ -1,7 +1,8 @@
-// pencil_kernels.cuh — the RK3 stage as four barrier-free sweeps (sm_100a).
+// pencil_kernels.cuh — the RK3 stage as sweeps along the grid axes (sm_100a).
 //
-// One stage of solver.jl:298-326 on a periodic grid, organised for latency hiding instead of
-// shared-memory tiling:
+// One stage of solver.jl:298-326, as k_prep (below), the sweeps and the finish.  In FP64 the
+// sweeps are one launch (sweep_kernels.cuh).  In mixed precision, and in the persistent batches
+// of either precision, they are organised for latency hiding instead of shared-memory tiling:
 //   k_prep      every ghosted point: shock sensor ϕ (schemes.jl:1-24) and the mass fractions
 //               Y = max(ρi / max(ρ, eps), 0) (thermo.jl:391-394) into a scratch array;
 //   k_pencil<2> z sweep, k_pencil<1> y sweep, k_pencil<0> x sweep: a warp owns a pencil of 32
@@ -16,8 +17,8 @@
 //   so its stores coalesce) finishes the stage: div (div.jl), RK3 combination (utils.jl:95-112),
 //   c2Prim with the Newton temperature (utils.jl:2-48, thermo.jl:231-282), the transport law of
 //   the new state, and the periodic ghost images.
-// Configurations (flame_rk_stage_tiled): 3 as above; 4 moves the finish into k_finish, one
-// thread per cell; 5 and 6 are 3 and 4 with each z / y sweep split into a flow sweep (the NS = 0
+// Configurations (flame_rk_stage_tiled) of the mixed path: 3 as above; 4 moves the finish into
+// k_finish, one thread per cell; 5 and 6 are 3 and 4 with each z / y sweep split into a flow sweep (the NS = 0
 // instance of the same kernel) and a species sweep (PART 2: species fluxes and the
 // enthalpy-diffusion term of the energy flux, with fewer slots and registers).  The flame_batch_*
 // persistent kernels at the end of the file run configuration 3 over many cases.
@@ -563,6 +564,8 @@ __device__ __forceinline__ void finish_cell(const Args<QT> &A, int g, int gx, in
             }
 }
 
+#include "sweep_kernels.cuh"
+
 // x sweep (lanes along x, every access coalesced); it is the last sweep.  FIN: it finishes the
 // stage itself (configuration 3); otherwise it adds its differences to R and k_finish follows
 // (configuration 4: the FP64 finish then runs at full occupancy, apart from the sweep's
@@ -634,7 +637,8 @@ __global__ void __launch_bounds__(Wpb<0>::value * 32) k_pencil_x(const __grid_co
 
 // The stage's finish for configuration 4: one thread per interior cell, x fastest, with the
 // complete right-hand side already in R (the x sweep summed it).
-template <int NS, typename QT, bool LAW2>
+// X3: the three sweeps' parts are apart (R, R2 and x_field), to be summed as (z + y) + x.
+template <int NS, typename QT, bool LAW2, bool X3 = false>
 __device__ __forceinline__ void finish_thread(const Args<QT> &A, const MixTables<NS, QT> *mt,
                                               int block) {
     const int c = block * 128 + threadIdx.x;
@@ -644,13 +648,16 @@ __device__ __forceinline__ void finish_thread(const Args<QT> &A, const MixTables
     const int g = gx + A.sy * gy + A.sz * gz;
     double rhs[5 + NS];
 #pragma unroll
-    for (int n = 0; n < 5 + NS; ++n) rhs[n] = A.R[g + n * A.np];
+    for (int n = 0; n < 5 + NS; ++n) {
+        if constexpr (X3) rhs[n] = (A.R[g + n * A.np] + A.R2[g + n * A.np]) + *x_field(A, n, g);
+        else rhs[n] = A.R[g + n * A.np];
+    }
     finish_cell<NS, QT, LAW2>(A, g, gx, gy, gz, rhs, mt);
 }
 
 template <int NS, typename QT>
 __global__ void __launch_bounds__(128) k_finish(const __grid_constant__ Args<QT> A) {
-    finish_thread<NS, QT, false>(A, nullptr, blockIdx.x);
+    finish_thread<NS, QT, false, sizeof(QT) == 8>(A, nullptr, blockIdx.x);
 }
 
 // The finish with the mixture-averaged law (law 2).  Its mixture rule needs up to 166 registers
@@ -661,7 +668,7 @@ __global__ void __launch_bounds__(128, 4) k_finish_mix(const __grid_constant__ A
     __shared__ MixTables<NS, QT> mt;
     mix_tables_fill<NS, QT>(A.th, A.tr, mt);
     __syncthreads();
-    finish_thread<NS, QT, true>(A, &mt, blockIdx.x);
+    finish_thread<NS, QT, true, sizeof(QT) == 8>(A, &mt, blockIdx.x);
 }
 
 // Columns per block of the staged y / z sweeps.  Single precision: 16 consecutive x columns, so
@@ -695,10 +702,6 @@ struct Staged {
         PART == 2 ? (sizeof(CT) * NSLOT * 33 * 16 <= 200 * 1024 ? 16 : 8)
                   : staged_cols(NS, sizeof(CT));
     static constexpr size_t SMEM = sizeof(CT) * STRIDE * COLS;
-    // three 8-column FP64 blocks per SM when their shared memory fits (228 KB per SM, 1 KB
-    // reserved per block): at most 80 registers; otherwise no bound
-    static constexpr int MINB =
-        (sizeof(CT) == 8 && COLS == 8 && 3 * (SMEM + 1024) <= 228 * 1024) ? 3 : 1;
 };
 
 // y or z sweep (DIR 1, 2).  The block stages the points of COLS neighbouring pencils with
@@ -814,16 +817,6 @@ __device__ __forceinline__ void staged_block(const Args<QT> &A, int block, unsig
 template <int DIR, int PASS, int NS, typename QT, typename CT, int PART = 0, bool MIXD = false>
 __global__ void __launch_bounds__(Staged<NS, CT, PART, MIXD>::COLS * 32)
     k_pencil_staged(const __grid_constant__ Args<QT> A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    staged_block<DIR, PASS, NS, QT, CT, PART, MIXD>(A, blockIdx.x, smem_raw);
-}
-
-// The same sweep held to the registers of three blocks per SM (Staged::MINB == 3).  A separate
-// kernel: naming a minimum of one block per SM changes the compiler's register choices against
-// leaving it out, so the other instances keep the plain bound above.
-template <int DIR, int PASS, int NS, typename QT, typename CT, int PART = 0, bool MIXD = false>
-__global__ void __launch_bounds__(Staged<NS, CT, PART, MIXD>::COLS * 32, 3)
-    k_pencil_staged3(const __grid_constant__ Args<QT> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     staged_block<DIR, PASS, NS, QT, CT, PART, MIXD>(A, blockIdx.x, smem_raw);
 }
@@ -1073,13 +1066,8 @@ int launch_staged(const Args<QT> &A, cudaStream_t s) {
     const int n_c2 = DIR == 1 ? A.nz : A.ny;
     const long long blocks = (long long)((A.nx + ST::COLS - 1) / ST::COLS) *
                              ((n_along + OWN - 1) / OWN) * n_c2;
-    if constexpr (ST::MINB == 3) {
-        if (int e = set_smem(k_pencil_staged3<DIR, PASS, NS, QT, CT, PART, MIXD>, sm, done)) return e;
-        k_pencil_staged3<DIR, PASS, NS, QT, CT, PART, MIXD><<<(unsigned)blocks, ST::COLS * 32, sm, s>>>(A);
-    } else {
-        if (int e = set_smem(k_pencil_staged<DIR, PASS, NS, QT, CT, PART, MIXD>, sm, done)) return e;
-        k_pencil_staged<DIR, PASS, NS, QT, CT, PART, MIXD><<<(unsigned)blocks, ST::COLS * 32, sm, s>>>(A);
-    }
+    if (int e = set_smem(k_pencil_staged<DIR, PASS, NS, QT, CT, PART, MIXD>, sm, done)) return e;
+    k_pencil_staged<DIR, PASS, NS, QT, CT, PART, MIXD><<<(unsigned)blocks, ST::COLS * 32, sm, s>>>(A);
     return flame_check_launch("flame_rk_stage (pencil)");
 }
 
@@ -1094,37 +1082,69 @@ int launch_x(const Args<QT> &A, cudaStream_t s) {
     return flame_check_launch("flame_rk_stage (pencil)");
 }
 
-template <int NS, typename QT, typename CT>
+// FP64: prep, the three sweeps in one launch, finish.
+template <int NS, bool MIXD>
+int launch_sweeps(const Args<double> &A, cudaStream_t s) {
+    constexpr size_t sm = SweepSlots<NS, MIXD>::SMEM;
+    static std::atomic<bool> done[64];
+    if (int e = set_smem(k_sweeps<NS, MIXD>, sm, done)) return e;
+    const SweepShape P = sweep_shape(A.nx, A.ny, A.nz);
+    k_sweeps<NS, MIXD><<<(unsigned)P.blocks, P.threads, sm, s>>>(A, P);
+    return flame_check_launch("flame_rk_stage (sweeps)");
+}
+template <int NS>
+int launch_fp64(const Args<double> &A, cudaStream_t s) {
+    k_prep<NS, double><<<(unsigned)((A.np + 255) / 256), 256, 0, s>>>(A);
+    if (int e = flame_check_launch("flame_rk_stage (prep)")) return e;
+    const unsigned blocks = (unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128);
+    // law 2: per-species D_k (one species has the one D of the other laws)
+    if (int e = A.tr.law == 2 ? launch_sweeps<NS, (NS > 1)>(A, s) : launch_sweeps<NS, false>(A, s))
+        return e;
+    if (A.tr.law == 2) k_finish_mix<NS, double><<<blocks, 128, 0, s>>>(A);
+    else k_finish<NS, double><<<blocks, 128, 0, s>>>(A);
+    return flame_check_launch("flame_rk_stage (finish)");
+}
+
+// Mixed precision: prep, z, y and x sweeps one after the other (see the top of this file).
+template <int NS>
+int launch_mixed(const Args<float> &A, cudaStream_t s, bool split_finish, bool split_species) {
+    using T = float;
+    k_prep<NS, T><<<(unsigned)((A.np + 255) / 256), 256, 0, s>>>(A);
+    if (int e = flame_check_launch("flame_rk_stage (prep)")) return e;
+    const unsigned blocks = (unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128);
+    if (A.tr.law == 2) {  // per-species D_k: configuration 6's launches with the MIXD sweeps
+        if (int e = launch_staged<2, 0, 0, T, T>(A, s)) return e;
+        if (int e = launch_staged<2, 0, NS, T, T, 2, true>(A, s)) return e;
+        if (int e = launch_staged<1, 1, 0, T, T>(A, s)) return e;
+        if (int e = launch_staged<1, 1, NS, T, T, 2, true>(A, s)) return e;
+        if (int e = launch_x<NS, T, T, false, true>(A, s)) return e;
+        k_finish_mix<NS, T><<<blocks, 128, 0, s>>>(A);
+        return flame_check_launch("flame_rk_stage (finish)");
+    }
+    if (split_species) {  // configurations 5, 6: flow sweep (the NS = 0 instance) + species sweep
+        if (int e = launch_staged<2, 0, 0, T, T>(A, s)) return e;
+        if (int e = launch_staged<2, 0, NS, T, T, 2>(A, s)) return e;
+        if (int e = launch_staged<1, 1, 0, T, T>(A, s)) return e;
+        if (int e = launch_staged<1, 1, NS, T, T, 2>(A, s)) return e;
+    } else {
+        if (int e = launch_staged<2, 0, NS, T, T>(A, s)) return e;
+        if (int e = launch_staged<1, 1, NS, T, T>(A, s)) return e;
+    }
+    if (!split_finish) return launch_x<NS, T, T, true>(A, s);
+    if (int e = launch_x<NS, T, T, false>(A, s)) return e;
+    k_finish<NS, T><<<blocks, 128, 0, s>>>(A);
+    return flame_check_launch("flame_rk_stage (finish)");
+}
+
+// The stage in the storage type QT.  FP64 runs the same three launches for every pencil
+// configuration; split_finish and split_species pick the mixed path's.
+template <int NS, typename QT>
 int launch(const FlameGrid &g, cudaStream_t s, int stage, double dt, const FlameStageBuffers &b,
            const FlameMetrics &m, const FlameThermo &th, const FlameTransport &tr,
            void *scratch, bool split_finish, bool split_species) {
     const Args<QT> A = make_args<QT>(g, stage, dt, b, m, th, tr, scratch);
-    k_prep<NS, QT><<<(unsigned)((A.np + 255) / 256), 256, 0, s>>>(A);
-    if (int e = flame_check_launch("flame_rk_stage (prep)")) return e;
-    if (tr.law == 2) {  // per-species D_k: configuration 6's launches with the MIXD sweeps
-        if (int e = launch_staged<2, 0, 0, QT, CT>(A, s)) return e;
-        if (int e = launch_staged<2, 0, NS, QT, CT, 2, true>(A, s)) return e;
-        if (int e = launch_staged<1, 1, 0, QT, CT>(A, s)) return e;
-        if (int e = launch_staged<1, 1, NS, QT, CT, 2, true>(A, s)) return e;
-        if (int e = launch_x<NS, QT, CT, false, true>(A, s)) return e;
-        k_finish_mix<NS, QT><<<(unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128), 128, 0,
-                               s>>>(A);
-        return flame_check_launch("flame_rk_stage (finish)");
-    }
-    if (split_species) {  // configurations 5, 6: flow sweep (the NS = 0 instance) + species sweep
-        if (int e = launch_staged<2, 0, 0, QT, CT>(A, s)) return e;
-        if (int e = launch_staged<2, 0, NS, QT, CT, 2>(A, s)) return e;
-        if (int e = launch_staged<1, 1, 0, QT, CT>(A, s)) return e;
-        if (int e = launch_staged<1, 1, NS, QT, CT, 2>(A, s)) return e;
-    } else {
-        if (int e = launch_staged<2, 0, NS, QT, CT>(A, s)) return e;
-        if (int e = launch_staged<1, 1, NS, QT, CT>(A, s)) return e;
-    }
-    if (!split_finish) return launch_x<NS, QT, CT, true>(A, s);
-    if (int e = launch_x<NS, QT, CT, false>(A, s)) return e;
-    const long long cells = (long long)A.nx * A.ny * A.nz;
-    k_finish<NS, QT><<<(unsigned)((cells + 127) / 128), 128, 0, s>>>(A);
-    return flame_check_launch("flame_rk_stage (finish)");
+    if constexpr (sizeof(QT) == 8) return launch_fp64<NS>(A, s);
+    else return launch_mixed<NS>(A, s, split_finish, split_species);
 }
 
 // ---------------------------------------------------------------- batches: one species count

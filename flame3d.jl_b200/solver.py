@@ -259,13 +259,17 @@ class DeviceCase:
         return self.tile
 
     def launches_per_stage(self) -> int:
-        """Kernels one fused stage launches: 4 for the pencil sweeps, one more with the
-        separate finish (4, 6) and two more with split species sweeps (5, 6); 1 for a tile
-        kernel."""
+        """Kernels one fused stage launches: 1 for a tile kernel, 3 for the pencil
+        configurations in FP64; in mixed precision 4, one more with the separate finish (4, 6)
+        and two more with split species sweeps (5, 6)."""
+        if self.precision == 0 and self.launched_config in (3, 4, 5, 6):
+            return 3
         return {3: 4, 4: 5, 5: 6, 6: 7}.get(self.launched_config, 1)
 
     def stage_kernels(self) -> str:
         t = self.launched_config
+        if t in (3, 4, 5, 6) and self.precision == 0:
+            return "pencil::k_prep + k_sweeps<z, y, x> + k_finish"
         if t in (3, 4, 5, 6):
             yz = ("k_pencil_staged<z> + k_pencil_staged<y>" if t < 5 else
                   "k_pencil_staged<z, flow> + k_pencil_staged<z, species> + "

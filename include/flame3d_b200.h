@@ -370,16 +370,18 @@ int flame_rk_stage(const FlameGrid *g, flame_stream_t stream, int stage, double 
                    const FlameTransport *transport, int precision);
 
 /* flame_rk_stage with an explicit configuration: 0, 1, 2 = one tile kernel per stage (16x8x8
- * with one CTA per SM, 16x8x8 with two, 8x8x8 with two); 3 = four barrier-free launches
- * (a prep pass and z, y, x warp-per-pencil sweeps, the x sweep finishing the stage) that need
- * b->scratch; 4 = configuration 3 with the finish (RK3 update, c2Prim, transport, ghosts) in a
- * fifth, per-cell launch, bit-identical to 3; 5, 6 = configurations 3, 4 with each y / z sweep
- * split into a flow sweep and a species sweep (fewer registers and shared-memory slots per
- * sweep when there are many species).  The autotuner picks the configuration per grid,
- * species count and precision.  Transport law 2 runs on configurations 3-6, always with
- * configuration 6's launches (its species sweeps and x sweep read each species' D_k, and the
- * finish evaluates the mixture rule per cell); configurations 0-2 refuse it with
- * FLAME_EUNSUPPORTED. */
+ * with one CTA per SM, 16x8x8 with two, 8x8x8 with two); 3 to 6 = sweeps along the grid axes that
+ * need b->scratch.  FP64 runs 3 to 6 as the same three launches: a prep pass, the z, y and x
+ * sweeps side by side, the finish (RK3 update, c2Prim, transport, ghosts); the interior of Q_out
+ * and rhoi_out holds the x sweep's part between the last two.  In mixed precision 3 = four
+ * barrier-free launches (a prep pass and z, y, x warp-per-pencil sweeps, the x sweep finishing
+ * the stage); 4 = configuration 3 with the finish in a fifth, per-cell launch, bit-identical to 3;
+ * 5, 6 = configurations 3, 4 with each z / y sweep split into a flow sweep and a species sweep
+ * (fewer registers and shared-memory slots per sweep when there are many species).  The
+ * autotuner picks the configuration per grid, species count and precision.  Transport law 2 runs
+ * on configurations 3-6, in mixed precision always with configuration 6's launches (its species
+ * sweeps and x sweep read each species' D_k, and the finish evaluates the mixture rule per cell);
+ * configurations 0-2 refuse it with FLAME_EUNSUPPORTED. */
 int flame_rk_stage_tiled(const FlameGrid *g, flame_stream_t stream, int stage, double dt,
                          const FlameStageBuffers *b, const FlameMetrics *m,
                          const FlameThermo *thermo, const FlameTransport *transport,
