@@ -353,7 +353,7 @@ struct Tile {
                 int x, y, z;
                 sweep_cell<DIR>(a, b, ch, x, y, z);
                 const int xl = x - (DIR == 0), yl = y - (DIR == 1), zl = z - (DIR == 2);
-                const CT phif = nmax(sPhi[b1i(xl, yl, zl)], sPhi[b1i(x, y, z)]);
+                const CT phif = CT(jmax(double(sPhi[b1i(xl, yl, zl)]), double(sPhi[b1i(x, y, z)])));
                 const int p0 = a + (LEN + 6) * b;  // point index of along-coordinate a-3
                 CT G[L::VG];
 #pragma unroll

@@ -1,8 +1,9 @@
 // pencil_kernels.cuh — the RK3 stage as sweeps along the grid axes (sm_100a).
 //
 // One stage of solver.jl:298-326, as k_prep (below), the sweeps and the finish.  In FP64 the
-// sweeps are one launch (sweep_kernels.cuh).  In mixed precision, and in the persistent batches
-// of either precision, they are organised for latency hiding instead of shared-memory tiling:
+// sweeps are one launch, in mixed precision most are (sweep_kernels.cuh).  The rest of the mixed
+// path (one species on large grids, law 2, configurations 5 and 6) and the persistent batches of
+// either precision are organised for latency hiding instead of shared-memory tiling:
 //   k_prep      every ghosted point: shock sensor ϕ (schemes.jl:1-24) and the mass fractions
 //               Y = max(ρi / max(ρ, eps), 0) (thermo.jl:391-394) into a scratch array;
 //   k_pencil<2> z sweep, k_pencil<1> y sweep, k_pencil<0> x sweep: a warp owns a pencil of 32
@@ -292,7 +293,7 @@ __device__ __forceinline__ void face_phase(const Args<QT> &A, const CT *S, int l
     const CT h = CT(0.5), c23 = CT(2.0 / 3.0), c12 = CT(1.0 / 12.0);
 #define SV(slot, ll) S[(slot) * 32 + (ll)]
     const int lm = l - 1;
-    const CT phif = nmax(SV(SL::PHI, lm), SV(SL::PHI, l));
+    const CT phif = CT(jmax(double(SV(SL::PHI, lm)), double(SV(SL::PHI, l))));
     auto recon = [&](int vp, int vm) {
         CT pv[7], mv[7];
 #pragma unroll
@@ -637,7 +638,7 @@ __global__ void __launch_bounds__(Wpb<0>::value * 32) k_pencil_x(const __grid_co
 
 // The stage's finish for configuration 4: one thread per interior cell, x fastest, with the
 // complete right-hand side already in R (the x sweep summed it).
-// X3: the three sweeps' parts are apart (R, R2 and x_field), to be summed as (z + y) + x.
+// X3: the three sweeps' parts are apart (R, R2 and get_x), to be summed as (z + y) + x.
 template <int NS, typename QT, bool LAW2, bool X3 = false>
 __device__ __forceinline__ void finish_thread(const Args<QT> &A, const MixTables<NS, QT> *mt,
                                               int block) {
@@ -649,15 +650,15 @@ __device__ __forceinline__ void finish_thread(const Args<QT> &A, const MixTables
     double rhs[5 + NS];
 #pragma unroll
     for (int n = 0; n < 5 + NS; ++n) {
-        if constexpr (X3) rhs[n] = (A.R[g + n * A.np] + A.R2[g + n * A.np]) + *x_field(A, n, g);
+        if constexpr (X3) rhs[n] = (A.R[g + n * A.np] + A.R2[g + n * A.np]) + get_x(A, n, g);
         else rhs[n] = A.R[g + n * A.np];
     }
     finish_cell<NS, QT, LAW2>(A, g, gx, gy, gz, rhs, mt);
 }
 
-template <int NS, typename QT>
+template <int NS, typename QT, bool X3>
 __global__ void __launch_bounds__(128) k_finish(const __grid_constant__ Args<QT> A) {
-    finish_thread<NS, QT, false, sizeof(QT) == 8>(A, nullptr, blockIdx.x);
+    finish_thread<NS, QT, false, X3>(A, nullptr, blockIdx.x);
 }
 
 // The finish with the mixture-averaged law (law 2).  Its mixture rule needs up to 166 registers
@@ -1088,7 +1089,7 @@ int launch_sweeps(const Args<double> &A, cudaStream_t s) {
     constexpr size_t sm = SweepSlots<NS, MIXD>::SMEM;
     static std::atomic<bool> done[64];
     if (int e = set_smem(k_sweeps<NS, MIXD>, sm, done)) return e;
-    const SweepShape P = sweep_shape(A.nx, A.ny, A.nz);
+    const SweepShape P = sweep_shape<SweepSlots<NS, MIXD>>(A.nx, A.ny, A.nz);
     k_sweeps<NS, MIXD><<<(unsigned)P.blocks, P.threads, sm, s>>>(A, P);
     return flame_check_launch("flame_rk_stage (sweeps)");
 }
@@ -1101,11 +1102,33 @@ int launch_fp64(const Args<double> &A, cudaStream_t s) {
     if (int e = A.tr.law == 2 ? launch_sweeps<NS, (NS > 1)>(A, s) : launch_sweeps<NS, false>(A, s))
         return e;
     if (A.tr.law == 2) k_finish_mix<NS, double><<<blocks, 128, 0, s>>>(A);
-    else k_finish<NS, double><<<blocks, 128, 0, s>>>(A);
+    else k_finish<NS, double, true><<<blocks, 128, 0, s>>>(A);
     return flame_check_launch("flame_rk_stage (finish)");
 }
 
-// Mixed precision: prep, z, y and x sweeps one after the other (see the top of this file).
+// Mixed precision: the sweeps of sweep_kernels.cuh.
+template <int NS>
+int launch_mixed_sweeps(const Args<float> &A, cudaStream_t s) {
+    using SL = MixedSlots<NS>;
+    static std::atomic<bool> done[64];
+    if (int e = set_smem(k_sweeps_mixed<NS>, SL::SMEM, done)) return e;
+    const SweepShape P = sweep_shape<SL>(A.nx, A.ny, A.nz);
+    const int first = SL::FIN ? P.x0 : P.blocks;
+    k_sweeps_mixed<NS><<<(unsigned)first, P.threads, SL::SMEM, s>>>(A, P);
+    if (int e = flame_check_launch("flame_rk_stage (sweeps)")) return e;
+    if constexpr (SL::FIN) {
+        static std::atomic<bool> done_x[64];
+        if (int e = set_smem(k_sweep_x_finish<NS>, SL::SMEM, done_x)) return e;
+        k_sweep_x_finish<NS><<<(unsigned)(P.blocks - P.x0), P.threads, SL::SMEM, s>>>(A, P);
+    } else {
+        k_finish<NS, float, true><<<(unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128), 128, 0,
+                                    s>>>(A);
+    }
+    return flame_check_launch("flame_rk_stage (finish)");
+}
+
+// Mixed precision: prep, then the sweeps (and, for law 2, configurations 5 and 6 and one species on
+// large grids, the staged sweeps one after the other; see the top of this file).
 template <int NS>
 int launch_mixed(const Args<float> &A, cudaStream_t s, bool split_finish, bool split_species) {
     using T = float;
@@ -1126,13 +1149,15 @@ int launch_mixed(const Args<float> &A, cudaStream_t s, bool split_finish, bool s
         if (int e = launch_staged<2, 0, NS, T, T, 2>(A, s)) return e;
         if (int e = launch_staged<1, 1, 0, T, T>(A, s)) return e;
         if (int e = launch_staged<1, 1, NS, T, T, 2>(A, s)) return e;
-    } else {
+    } else if (NS > 1 || !staged_sweeps_ahead(NS, (long long)A.nx * A.ny * A.nz)) {
+        return launch_mixed_sweeps<NS>(A, s);  // configurations 3, 4
+    } else if constexpr (NS == 1) {
         if (int e = launch_staged<2, 0, NS, T, T>(A, s)) return e;
         if (int e = launch_staged<1, 1, NS, T, T>(A, s)) return e;
     }
     if (!split_finish) return launch_x<NS, T, T, true>(A, s);
     if (int e = launch_x<NS, T, T, false>(A, s)) return e;
-    k_finish<NS, T><<<blocks, 128, 0, s>>>(A);
+    k_finish<NS, T, false><<<blocks, 128, 0, s>>>(A);
     return flame_check_launch("flame_rk_stage (finish)");
 }
 

@@ -23,13 +23,13 @@
 // Tried and not kept: two blocks per SM at 128 registers (jet 6623) and four at 64 (7810);
 // everything but the metrics staged in pass 1 (6920); a prefetch of pass 2's lines to L2 (6399).
 
-constexpr int kSweepNT = 256;  // most threads (points) of a block, and the pitch of a slot
-constexpr int kSweepCols = 8;  // x columns of a y / z block
 
 // Slots of a point.  Passes 2 and 3 are one where its slots leave room for three blocks per SM
 // (ONE: up to three species, two with per-species D); the sensor keeps the last slot.
 template <int NS, bool MIXD>
 struct SweepSlots {
+    // x columns of a y / z block; most points of a block (its threads) and pitch of a slot
+    static constexpr int C = 8, NT = 32 * C, MINB = 3;
     static constexpr int FM = 5, SP = 10, SM = 10 + NS, F = 10 + 2 * NS;  // pass 1: F+ at 0
     static constexpr int YN = (MIXD ? 4 : 3) * NS;
     static constexpr int MOST = 37;
@@ -39,8 +39,8 @@ struct SweepSlots {
     static constexpr int a = F > 26 ? F : 26, b = a > YN ? a : YN;
     static constexpr int PHI = ONE ? Y + YN : b;
     static constexpr int N = PHI + 1;
-    static constexpr size_t SMEM = sizeof(double) * N * kSweepNT;
-    static_assert(N <= MOST && 3 * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
+    static constexpr size_t SMEM = sizeof(double) * N * NT;
+    static_assert(N <= MOST && MINB * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
 };
 
 // How the launch is cut: own cells per line and direction, lines per x block, threads per
@@ -50,11 +50,54 @@ struct SweepShape {
 };
 
 // Where the x sweep leaves field n of a cell for the finish: the stage's output arrays, whose
-// interior the finish of the same cell writes after it has read this (Q_out holds seven fields
-// of 8 bytes, rhoi_out one per species).
-__device__ __forceinline__ double *x_field(const Args<double> &A, int n, int c) {
-    return n < 5 ? A.Qo + n * A.np + c : A.ro + (n - 5) * A.np + c;
+// interior the finish of the same cell writes after it has read this (rhoi_out one value of 8
+// bytes per species; for the five flow fields Q_out's seven).
+__device__ __forceinline__ void put_x(const Args<double> &A, int n, int c, double d) {
+    (n < 5 ? A.Qo + n * A.np : A.ro + (n - 5) * A.np)[c] = d;
 }
+__device__ __forceinline__ double get_x(const Args<double> &A, int n, int c) {
+    return (n < 5 ? A.Qo + n * A.np : A.ro + (n - 5) * A.np)[c];
+}
+
+// A block's lines and a thread's place in them: its point, its face (left of a cell) and the
+// slot of the face's right cell.
+template <int DIR, int C>
+struct SweepPlace {
+    static constexpr int STEP = DIR == 0 ? 1 : C;  // the slot distance of two points of a line
+    int sy, sz, ng, ny, line_end;  // strides, ghosts; the last line in the grid
+    int first, other;              // first line (row, or x column); the third axis' position
+    int c0, cells;                 // first cell along the sweep, and how many
+    bool point, face;
+    int g, pf, fi, fl;             // the point; the face's slot, line and position
+    template <typename QT>
+    __device__ __forceinline__ SweepPlace(const Args<QT> &A, const SweepShape &P, int bid)
+        : sy(A.sy), sz(A.sz), ng(A.ng), ny(A.ny) {
+        const int tid = threadIdx.x;
+        const int n_along = DIR == 0 ? A.nx : DIR == 1 ? A.ny : A.nz;
+        const int own = P.own[DIR], L = own + 6, F = own + 1;
+        const int nseg = (n_along + own - 1) / own, seg = bid % nseg;
+        bid /= nseg;
+        c0 = seg * own, cells = min(own, n_along - c0);
+        const int nxb = (A.nx + C - 1) / C, lines = DIR == 0 ? P.rows : C;
+        first = DIR == 0 ? bid * P.rows : (bid % nxb) * C;
+        other = DIR == 0 ? 0 : bid / nxb;
+        line_end = DIR == 0 ? A.ny * A.nz - 1 : A.nx - 1;
+        const int li = DIR == 0 ? tid / L : tid % C, l = DIR == 0 ? tid % L : tid / C;
+        point = DIR == 0 ? li < lines : l < L;
+        g = at(min(li, lines - 1), min(c0 + ng - 3 + l, n_along + 2 * ng - 1));
+        fi = DIR == 0 ? tid / F : tid % C, fl = (DIR == 0 ? tid % F : tid / C) + 3;
+        face = fi < lines && first + fi <= line_end && fl <= cells + 3;
+        pf = face ? (DIR == 0 ? fi * L + fl : tid + 3 * C) : 3 * STEP;
+    }
+    // ghosted index of ghosted position a along the sweep of the block's line i, kept in the grid
+    __device__ __forceinline__ int at(int i, int a) const {
+        const int k = min(first + i, line_end);
+        if constexpr (DIR == 0) return a + sy * (k % ny + ng) + sz * (k / ny + ng);
+        else return k + ng + (DIR == 1 ? sy * a + sz * (other + ng) : sz * a + sy * (other + ng));
+    }
+    __device__ __forceinline__ bool cell() const { return face && fl < cells + 3; }
+    __device__ __forceinline__ int cell_index() const { return at(fi, c0 + ng - 3 + fl); }
+};
 
 // ---- faces: fluxes contracted with the face normal.
 // With md the metric row of the face direction and c_a = Σ_x met[a][x] md[x], a derivative
@@ -100,52 +143,22 @@ __device__ __forceinline__ double tangent4(const double *q, int s) {
     return 2.0 / 3.0 * (q[s] - q[-s]) - 1.0 / 12.0 * (q[2 * s] - q[-2 * s]);
 }
 
-// One block of a sweep.  STEP: the slot distance of two points of a line.
+// One block of an FP64 sweep.
 template <int DIR, int NS, bool MIXD>
 __device__ __forceinline__ void sweep_block(const Args<double> &A, const SweepShape &P, int bid,
                                             double *S) {
     using SL = SweepSlots<NS, MIXD>;
-    constexpr int NT = kSweepNT, C = kSweepCols, STEP = DIR == 0 ? 1 : C;
-    constexpr int D1 = Dir<DIR>::D1, D2 = Dir<DIR>::D2;
-    const int np = A.np, tid = threadIdx.x;
+    constexpr int NT = SL::NT, D1 = Dir<DIR>::D1, D2 = Dir<DIR>::D2;
+    using Place = SweepPlace<DIR, SL::C>;
+    constexpr int STEP = Place::STEP;
+    const Place W(A, P, bid);
+    const int np = A.np, g = W.g, pf = W.pf;
+    const bool point = W.point, face = W.face;
     const int stride[3] = {1, A.sy, A.sz};
-    const int st = stride[DIR], s1 = stride[D1], s2 = stride[D2];
+    const int s1 = stride[D1], s2 = stride[D2];
     const double *Q = A.Qi;
-    const int n_along = DIR == 0 ? A.nx : DIR == 1 ? A.ny : A.nz;
-    const int own = P.own[DIR], L = own + 6;
-    const int nseg = (n_along + own - 1) / own;
-    // the block's lines: its first cell along the sweep, and the interior position of a line
-    const int seg = bid % nseg;
-    bid /= nseg;
-    const int c0 = seg * own, cells = min(own, n_along - c0);
-    const int nxb = (A.nx + C - 1) / C;
-    const int xb = DIR == 0 ? 0 : (bid % nxb) * C, other = DIR == 0 ? 0 : bid / nxb;
-    const int row0 = DIR == 0 ? bid * P.rows : 0;
-    const int all_rows = A.ny * A.nz;
-    const int lines = DIR == 0 ? P.rows : C;
-    // ghosted index of position a (ghosted, along the sweep) of line i, clamped into the grid
-    auto at = [&](int i, int a) {
-        if constexpr (DIR == 0) {
-            const int r = min(row0 + i, all_rows - 1);
-            return a + A.sy * (r % A.ny + A.ng) + A.sz * (r / A.ny + A.ng);
-        } else {
-            const int x = min(xb + i, A.nx - 1) + A.ng;
-            return x + (DIR == 1 ? A.sy * a + A.sz * (other + A.ng) : A.sz * a + A.sy * (other + A.ng));
-        }
-    };
-    const int last = n_along + 2 * A.ng - 1;
-    // the thread's point, its face (left of the cell) and the face's slot
-    const int li = DIR == 0 ? tid / L : tid % C, l = DIR == 0 ? tid % L : tid / C;
-    const bool point = DIR == 0 ? li < lines : l < L;
-    const int g = at(min(li, lines - 1), min(c0 + A.ng - 3 + l, last));
-    const int F = own + 1;
-    const int fi = DIR == 0 ? tid / F : tid % C, fl = (DIR == 0 ? tid % F : tid / C) + 3;
-    const bool inside = DIR == 0 ? fi < lines && row0 + fi < all_rows
-                                 : xb + fi < A.nx;
-    const bool face = inside && fl <= cells + 3;
-    const int pf = DIR == 0 ? fi * L + fl : tid + 3 * C;
-    double *own_slot = S + tid;        // the point's slots
-    const double *f = S + (face ? pf : 3 * STEP);  // the face's right cell
+    double *own_slot = S + threadIdx.x;  // the point's slots
+    const double *f = S + pf;            // the face's right cell
 #define SV(slot, o) f[(slot) * NT + (o) * STEP]
 #define SUM(slot) (SV(slot, -1) + SV(slot, 0))
     auto stage_flow = [&]() {  // velocities, T, their tangential derivatives, transport
@@ -290,12 +303,12 @@ __device__ __forceinline__ void sweep_block(const Args<double> &A, const SweepSh
         for (int n = 0; n < 5 + NS; ++n) S[n * NT + pf] = G[n];
     }
     __syncthreads();
-    if (face && fl < cells + 3) {
-        const int gc = at(fi, c0 + A.ng - 3 + fl);
+    if (W.cell()) {
+        const int gc = W.cell_index();
 #pragma unroll
         for (int n = 0; n < 5 + NS; ++n) {
             const double d = G[n] - S[n * NT + pf + STEP];
-            if constexpr (DIR == 0) *x_field(A, n, gc) = d;
+            if constexpr (DIR == 0) put_x(A, n, gc, d);
             else (DIR == 2 ? A.R : A.R2)[gc + n * np] = d;
         }
     }
@@ -304,7 +317,7 @@ __device__ __forceinline__ void sweep_block(const Args<double> &A, const SweepSh
 }
 
 template <int NS, bool MIXD>
-__global__ void __launch_bounds__(kSweepNT, 3)
+__global__ void __launch_bounds__(SweepSlots<NS, MIXD>::NT, SweepSlots<NS, MIXD>::MINB)
     k_sweeps(const __grid_constant__ Args<double> A, const __grid_constant__ SweepShape P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *S = reinterpret_cast<double *>(smem_raw);
@@ -313,33 +326,312 @@ __global__ void __launch_bounds__(kSweepNT, 3)
     else if (b < P.x0) sweep_block<1, NS, MIXD>(A, P, b - P.y0, S);
     else sweep_block<0, NS, MIXD>(A, P, b - P.x0, S);
 }
+// ---- mixed precision.
+// The same passes in FP32, with the arithmetic of face_phase operation by operation (its results
+// to the last bit: a face whose sensor lies at a branch threshold follows every rounding of the
+// state), and the differences of two faces formed in FP64.  Up to two species the x sweep is a
+// launch of its own that finishes the stage; more species' finish would not fit its registers.
+//
+// Bound by issue (64x48x40 to 128x64x64 jets: 0.66 instructions per scheduler and cycle, 2378
+// slots per cell and sweep against 2874 of the staged sweeps).  One step, staged sweeps -> these:
+// 64^3 with one, two, three species 345 -> 307, 489 -> 382, 579 -> 441 us; 96^3 with four 1387 ->
+// 1151; 128^3 with two 2298 -> 2114; 192^3 with nine 18.1 -> 16.1 ms.  With one species on large
+// grids the staged sweeps stay ahead (96^3 756 / 758 us, 128^3 1584 / 1719, jet 256x128x128 4305 /
+// 4449), so from 2^20 cells on they are launched (staged_sweeps_ahead below).  Tried and not kept:
+// face fluxes in slots of their own, one barrier less (nine species at 192^3 16.1 -> 19.3 ms: the
+// shared memory comes out of L1); blocks in another order (within 2 %).
 
-// Cuts a launch.  y and z: eight columns of n / nseg cells, at most 26 (the points of a block
-// are 8 (own + 6) <= 256).  x: the rows per block and the cut of a row that need the fewest warps
+// Slots of a point in FP32.  ONE: everything in one pass, where two blocks of 512 threads fit an
+// SM with it (up to three species); otherwise all but the split fluxes in a second pass.  A
+// point's four-byte values fill half a line with sixteen columns, which serves best until the
+// species' registers spill at two blocks of 512 threads: from eight species on, three blocks of
+// 256 with eight columns (80 registers instead of 64).
+template <int NS>
+struct MixedSlots {
+    static constexpr int C = NS < 8 ? 16 : 8, NT = 32 * C, MINB = NS < 8 ? 2 : 3;
+    static constexpr int FM = 5, SP = 10, SM = 10 + NS, F = 10 + 2 * NS, M = 26 + 3 * NS;
+    static constexpr bool ONE = MINB * (sizeof(float) * (F + M + 1) * NT + 1024) <= 228 * 1024;
+    static constexpr int MET = ONE ? F : 0, Q4 = MET + 10, DQ1 = MET + 14, DQ2 = MET + 18, TR = MET + 22,
+                         RHO = MET + 25, Y = MET + 26, DY1 = Y + NS, DY2 = Y + 2 * NS,
+                         PHI = Y + 3 * NS, N = PHI + 1;
+    static_assert(N > F, "the sensor's slot is not the split fluxes'");
+    static constexpr size_t SMEM = sizeof(float) * N * NT;
+    // up to two species the finish fits the x sweep's 64 registers
+    static constexpr bool FIN = NS <= 2;
+};
+
+// The x sweep's FP64 flow differences as pairs of 32-bit words in Q_out's seven fields and the
+// transport's three.
+__device__ __forceinline__ int *x_word(const Args<float> &A, int k, int c) {
+    return reinterpret_cast<int *>(k < 7 ? A.Qo + k * A.np + c : A.To + (k - 7) * A.np + c);
+}
+__device__ __forceinline__ void put_x(const Args<float> &A, int n, int c, double d) {
+    if (n < 5) *x_word(A, 2 * n, c) = __double2loint(d), *x_word(A, 2 * n + 1, c) = __double2hiint(d);
+    else A.ro[(n - 5) * A.np + c] = d;
+}
+__device__ __forceinline__ double get_x(const Args<float> &A, int n, int c) {
+    return n < 5 ? __hiloint2double(*x_word(A, 2 * n + 1, c), *x_word(A, 2 * n, c))
+                 : A.ro[(n - 5) * A.np + c];
+}
+
+// FIN (x): the thread finishes its cell itself, with the z and y sweeps' parts from memory.
+template <int DIR, int NS, bool FIN = false>
+__device__ __forceinline__ void mixed_block(const Args<float> &A, const SweepShape &P, int bid,
+                                            float *S) {
+    using SL = MixedSlots<NS>;
+    constexpr int NT = SL::NT, D1 = Dir<DIR>::D1, D2 = Dir<DIR>::D2;
+    using Place = SweepPlace<DIR, SL::C>;
+    constexpr int STEP = Place::STEP;
+    const Place W(A, P, bid);
+    const int np = A.np, g = W.g, pf = W.pf;
+    const int stride[3] = {1, A.sy, A.sz};
+    const int s1 = stride[D1], s2 = stride[D2];
+    const float *Q = A.Qi;
+    float *own_slot = S + threadIdx.x;
+    const float *f = S + pf;
+    const float h = 0.5f, c23 = float(2.0 / 3.0), c12 = float(1.0 / 12.0);
+    auto metric = [&](int k) { return A.metq ? __ldg(A.metq + k * np + g) : float(__ldg(A.met[k] + g)); };
+    auto stage_rest = [&]() {
+#pragma unroll
+        for (int k = 0; k < 10; ++k) own_slot[(SL::MET + k) * NT] = metric(k);
+        const int qv[4] = {1, 2, 3, 5};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float *q = Q + qv[k] * np + g;
+            own_slot[(SL::Q4 + k) * NT] = q[0];
+            own_slot[(SL::DQ1 + k) * NT] = c23 * (q[s1] - q[-s1]) - c12 * (q[2 * s1] - q[-2 * s1]);
+            own_slot[(SL::DQ2 + k) * NT] = c23 * (q[s2] - q[-s2]) - c12 * (q[2 * s2] - q[-2 * s2]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) own_slot[(SL::TR + k) * NT] = A.Ti[g + k * np];
+        own_slot[SL::RHO * NT] = Q[g];
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+            const float *Y = A.aux + (1 + n) * np + g;
+            own_slot[(SL::Y + n) * NT] = Y[0];
+            own_slot[(SL::DY1 + n) * NT] = Y[s1] - Y[-s1];
+            own_slot[(SL::DY2 + n) * NT] = Y[s2] - Y[-s2];
+        }
+    };
+#define SV(slot, o) f[(slot) * NT + (o) * STEP]
+    if (W.point) {
+        float fp[5], fm[5];
+        const float E1 = split_fast(Q[g], Q[g + np], Q[g + 2 * np], Q[g + 3 * np], Q[g + 4 * np],
+                                    Q[g + 6 * np], metric(3 * DIR), metric(3 * DIR + 1),
+                                    metric(3 * DIR + 2), fp, fm);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) own_slot[n * NT] = fp[n], own_slot[(SL::FM + n) * NT] = fm[n];
+        const float Ep = h * (E1 + fabs(E1)), Em = h * (E1 - fabs(E1));
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+            const float r = float(A.ri[g + n * np]);
+            own_slot[(SL::SP + n) * NT] = Ep * r, own_slot[(SL::SM + n) * NT] = Em * r;
+        }
+        own_slot[SL::PHI * NT] = A.aux[g];
+        if constexpr (SL::ONE) stage_rest();
+    }
+    __syncthreads();
+    float G[5 + NS];
+    if (W.face) {
+        const float phif = nmax(SV(SL::PHI, -1), SV(SL::PHI, 0));
+        if constexpr (NS >= 8) {
+            // the branch outside the loop over the fields (192^3, nine species: 16.99 -> 16.07 ms
+            // a step; with fewer species the longer code costs 1-3 %); the sums of the two
+            // directions are kept apart from the products before them, as hybrid_face_fast's are
+            auto P = [&](int n, int o) { return SV(n < 5 ? n : SL::SP + n - 5, o); };
+            auto M = [&](int n, int o) { return SV(n < 5 ? SL::FM + n : SL::SM + n - 5, o); };
+            if (phif < float(kHybrid1)) {
+#pragma unroll
+                for (int n = 0; n < 5 + NS; ++n) {
+                    const float fp = float(kUP7_2) * P(n, -3) + float(kUP7_3) * P(n, -2) +
+                                     float(kUP7_4) * P(n, -1) + float(kUP7_5) * P(n, 0) +
+                                     float(kUP7_6) * P(n, 1) + float(kUP7_7) * P(n, 2);
+                    const float fm = float(kUP7_7) * M(n, -3) + float(kUP7_6) * M(n, -2) +
+                                     float(kUP7_5) * M(n, -1) + float(kUP7_4) * M(n, 0) +
+                                     float(kUP7_3) * M(n, 1) + float(kUP7_2) * M(n, 2);
+                    G[n] = __fadd_rn(fp, fm);
+                }
+            } else if (phif < float(kHybrid2)) {
+#pragma unroll
+                for (int n = 0; n < 5 + NS; ++n)
+                    G[n] = __fadd_rn(wenoz_plus_fast(P(n, -3), P(n, -2), P(n, -1), P(n, 0), P(n, 1)),
+                                     wenoz_minus_fast(M(n, -2), M(n, -1), M(n, 0), M(n, 1), M(n, 2)));
+            } else {
+#pragma unroll
+                for (int n = 0; n < 5 + NS; ++n) {
+                    const float p2 = P(n, -1), m3 = M(n, 0);
+                    const float fp = p2 + 0.5f * minmod(P(n, 0) - p2, p2 - P(n, -2));
+                    const float fm = m3 - 0.5f * minmod(M(n, 1) - m3, m3 - M(n, -1));
+                    G[n] = __fadd_rn(fp, fm);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < 5 + NS; ++n) {
+                const int vp = n < 5 ? n : SL::SP + n - 5, vm = n < 5 ? SL::FM + n : SL::SM + n - 5;
+                float p[7], m[7];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) p[i] = SV(vp, i - 3), m[i] = SV(vm, i - 3);
+                p[6] = m[6] = 0;
+                G[n] = hybrid_face_fast<float>(p, m, phif);
+            }
+        }
+    }
+    if constexpr (!SL::ONE) {
+        __syncthreads();
+        if (W.point) stage_rest();
+        __syncthreads();
+    }
+    if (W.face) {
+        float met[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) met[k] = (SV(SL::MET + k, -1) + SV(SL::MET + k, 0)) * h;
+        const float Jac = (SV(SL::MET + 9, -1) + SV(SL::MET + 9, 0)) * h;
+        const float DL = SV(SL::TR + 2, -1), DR = SV(SL::TR + 2, 0);
+        const float rho = (SV(SL::RHO, -1) + SV(SL::RHO, 0)) * h;
+        const float Tf = (SV(SL::Q4 + 3, -1) + SV(SL::Q4 + 3, 0)) * h;
+        const float *md = met + 3 * DIR;
+        const float rhoDi = (DL + DR) * rho;  // viscous.jl:473 (no 1/2, as the reference)
+        auto diffusion = [&](int n, float &Vx, float &Vy, float &Vz) {
+            const float y0 = SV(SL::Y + n, 0), ym = SV(SL::Y + n, -1);
+            const float yp = SV(SL::Y + n, 1), ymm = SV(SL::Y + n, -2);
+            float dY[3];
+            dY[DIR] = 1.25f * (y0 - ym) - c12 * (yp - ymm);
+            dY[D1] = 0.25f * (SV(SL::DY1 + n, 0) + SV(SL::DY1 + n, -1));
+            dY[D2] = 0.25f * (SV(SL::DY2 + n, 0) + SV(SL::DY2 + n, -1));
+            Vx = (dY[0] * met[0] + dY[1] * met[3] + dY[2] * met[6]) * Jac * rhoDi;
+            Vy = (dY[0] * met[1] + dY[1] * met[4] + dY[2] * met[7]) * Jac * rhoDi;
+            Vz = (dY[0] * met[2] + dY[1] * met[5] + dY[2] * met[8]) * Jac * rhoDi;
+            return h * (ym + y0);
+        };
+        float sum1 = 0, sum2 = 0, sum3 = 0;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+            float Vx, Vy, Vz;
+            diffusion(n, Vx, Vy, Vz);
+            sum1 += Vx, sum2 += Vy, sum3 += Vz;
+        }
+        float fh1 = 0, fh2 = 0, fh3 = 0;
+        {
+            const double Td = double(Tf);
+            const double T2 = 0.5 * Td * Td, T3 = 2.0 / 3.0 * T2 * Td, T4 = T2 * T2, T5 = 0.8 * T4 * Td;
+#pragma unroll
+            for (int n = 0; n < NS; ++n) {
+                float Vx, Vy, Vz;
+                const float Yf = diffusion(n, Vx, Vy, Vz);
+                const float hn = float(h_spec(A.th, n, Td, T2, T3, T4, T5));
+                const float V1 = Vx - sum1 * Yf, V2 = Vy - sum2 * Yf, V3 = Vz - sum3 * Yf;
+                G[5 + n] = G[5 + n] - (V1 * md[0] + V2 * md[1] + V3 * md[2]);
+                fh1 += V1 * hn, fh2 += V2 * hn, fh3 += V3 * hn;
+            }
+        }
+        const float mui = (SV(SL::TR, -1) + SV(SL::TR, 0)) * h;
+        const float lami = (SV(SL::TR + 1, -1) + SV(SL::TR + 1, 0)) * h;
+        // momentum and energy, viscous.jl:14-141
+        float gr[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float dq[3];
+            dq[DIR] = 1.25f * (SV(SL::Q4 + k, 0) - SV(SL::Q4 + k, -1)) -
+                      c12 * (SV(SL::Q4 + k, 1) - SV(SL::Q4 + k, -2));
+            dq[D1] = h * (SV(SL::DQ1 + k, 0) + SV(SL::DQ1 + k, -1));
+            dq[D2] = h * (SV(SL::DQ2 + k, 0) + SV(SL::DQ2 + k, -1));
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+                gr[k][x] = (dq[0] * met[x] + dq[1] * met[3 + x] + dq[2] * met[6 + x]) * Jac;
+        }
+        const float u = (SV(SL::Q4 + 0, -1) + SV(SL::Q4 + 0, 0)) * h;
+        const float v = (SV(SL::Q4 + 1, -1) + SV(SL::Q4 + 1, 0)) * h;
+        const float w = (SV(SL::Q4 + 2, -1) + SV(SL::Q4 + 2, 0)) * h;
+        const float div = gr[0][0] + gr[1][1] + gr[2][2];
+        const float t11 = mui * (2 * gr[0][0] - c23 * div);
+        const float t12 = mui * (gr[0][1] + gr[1][0]);
+        const float t13 = mui * (gr[0][2] + gr[2][0]);
+        const float t22 = mui * (2 * gr[1][1] - c23 * div);
+        const float t23 = mui * (gr[2][1] + gr[1][2]);
+        const float t33 = mui * (2 * gr[2][2] - c23 * div);
+        const float E1 = u * t11 + v * t12 + w * t13 + lami * gr[3][0] + fh1;
+        const float E2 = u * t12 + v * t22 + w * t23 + lami * gr[3][1] + fh2;
+        const float E3 = u * t13 + v * t23 + w * t33 + lami * gr[3][2] + fh3;
+        G[1] -= md[0] * t11 + md[1] * t12 + md[2] * t13;
+        G[2] -= md[0] * t12 + md[1] * t22 + md[2] * t23;
+        G[3] -= md[0] * t13 + md[1] * t23 + md[2] * t33;
+        G[4] -= md[0] * E1 + md[1] * E2 + md[2] * E3;
+    }
+#undef SV
+    __syncthreads();
+    if (W.face) {
+#pragma unroll
+        for (int n = 0; n < 5 + NS; ++n) S[n * NT + pf] = G[n];
+    }
+    __syncthreads();
+    if (W.cell()) {
+        const int gc = W.cell_index();
+        double rhs[FIN ? 5 + NS : 1];
+#pragma unroll
+        for (int n = 0; n < 5 + NS; ++n) {
+            const double d = double(G[n]) - double(S[n * NT + pf + STEP]);
+            if constexpr (FIN) rhs[n] = (A.R[gc + n * np] + A.R2[gc + n * np]) + d;
+            else if constexpr (DIR == 0) put_x(A, n, gc, d);
+            else (DIR == 2 ? A.R : A.R2)[gc + n * np] = d;
+        }
+        if constexpr (FIN) {
+            const int gy = gc / A.sy;
+            finish_cell<NS>(A, gc, gc - gy * A.sy, gy % A.ty, gy / A.ty, rhs);
+        }
+    }
+}
+
+template <int NS>
+__global__ void __launch_bounds__(MixedSlots<NS>::NT, MixedSlots<NS>::MINB)
+    k_sweeps_mixed(const __grid_constant__ Args<float> A, const __grid_constant__ SweepShape P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float *S = reinterpret_cast<float *>(smem_raw);
+    const int b = blockIdx.x;
+    if (b < P.y0) mixed_block<2, NS>(A, P, b, S);
+    else if (b < P.x0) mixed_block<1, NS>(A, P, b - P.y0, S);
+    else mixed_block<0, NS>(A, P, b - P.x0, S);
+}
+// The x sweep that finishes the stage (after k_sweeps_mixed of the other two directions).
+template <int NS>
+__global__ void __launch_bounds__(MixedSlots<NS>::NT, MixedSlots<NS>::MINB)
+    k_sweep_x_finish(const __grid_constant__ Args<float> A, const __grid_constant__ SweepShape P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    mixed_block<0, NS, true>(A, P, blockIdx.x, reinterpret_cast<float *>(smem_raw));
+}
+
+// Cuts a launch.  y and z: C columns of n / nseg cells, at most 26 (the points of a block are
+// C (own + 6) <= 32 C).  x: the rows per block and the cut of a row that need the fewest warps
 // (those of the points and those of the faces) per cell.
+template <typename SL>
 inline SweepShape sweep_shape(int nx, int ny, int nz) {
+    constexpr int C = SL::C, NT = SL::NT;
     SweepShape P{};
-    const int most = kSweepNT / kSweepCols - 6;
+    const int most = NT / C - 6;
     const int ext[3] = {nx, ny, nz};
     for (int d = 1; d < 3; ++d) {
         const int nseg = (ext[d] + most - 1) / most;
         P.own[d] = (ext[d] + nseg - 1) / nseg;
     }
+    const long long all = ny * (long long)nz;
     double best = 1e300;
     for (int nseg = 1; nseg <= (nx + 25) / 26 + 1; ++nseg) {
         const int own = (nx + nseg - 1) / nseg;
-        for (int rows = 1; rows * (own + 6) <= kSweepNT; ++rows) {
+        for (int rows = 1; rows * (own + 6) <= NT; ++rows) {
             const double warps = (rows * (own + 6) + 31) / 32 + (rows * (own + 1) + 31) / 32;
-            const double blocks = double((ny * (long long)nz + rows - 1) / rows) * ((nx + own - 1) / own);
+            const double blocks = double((all + rows - 1) / rows) * ((nx + own - 1) / own);
             if (warps * blocks < best) best = warps * blocks, P.own[0] = own, P.rows = rows;
         }
     }
-    const int nxb = (nx + kSweepCols - 1) / kSweepCols;
+    const int nxb = (nx + C - 1) / C;
     P.y0 = nxb * ny * ((nz + P.own[2] - 1) / P.own[2]);
     P.x0 = P.y0 + nxb * nz * ((ny + P.own[1] - 1) / P.own[1]);
-    P.blocks = P.x0 + (int)((ny * (long long)nz + P.rows - 1) / P.rows) * ((nx + P.own[0] - 1) / P.own[0]);
+    P.blocks = P.x0 + (int)((all + P.rows - 1) / P.rows) * ((nx + P.own[0] - 1) / P.own[0]);
     int t = P.rows * (P.own[0] + 6);
-    for (int d = 1; d < 3; ++d) t = t > kSweepCols * (P.own[d] + 6) ? t : kSweepCols * (P.own[d] + 6);
+    for (int d = 1; d < 3; ++d) t = t > C * (P.own[d] + 6) ? t : C * (P.own[d] + 6);
     P.threads = (t + 31) / 32 * 32;
     return P;
 }
+
+// Mixed precision: one species on at least 2^20 cells runs the staged sweeps (figures above).
+inline bool staged_sweeps_ahead(int ns, long long cells) { return ns == 1 && cells >= 1 << 20; }

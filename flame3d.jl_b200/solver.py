@@ -258,18 +258,30 @@ class DeviceCase:
             return 6
         return self.tile
 
+    @property
+    def swept(self) -> bool:
+        """Whether a pencil configuration runs the sweeps of sweep_kernels.cuh: all of FP64; in
+        mixed precision configurations 3 and 4 but for one species on at least 2^20 cells."""
+        t = self.launched_config
+        if self.precision == 0:
+            return t in (3, 4, 5, 6)
+        return t in (3, 4) and (self.case.ns > 1 or self.case.cells < 1 << 20)
+
     def launches_per_stage(self) -> int:
-        """Kernels one fused stage launches: 1 for a tile kernel, 3 for the pencil
-        configurations in FP64; in mixed precision 4, one more with the separate finish (4, 6)
-        and two more with split species sweeps (5, 6)."""
-        if self.precision == 0 and self.launched_config in (3, 4, 5, 6):
+        """Kernels one fused stage launches: 1 for a tile kernel, 3 for the sweeps in one launch;
+        with the staged sweeps 4, one more with the separate finish (4, 6) and two more with
+        split species sweeps (5, 6)."""
+        if self.swept:
             return 3
         return {3: 4, 4: 5, 5: 6, 6: 7}.get(self.launched_config, 1)
 
     def stage_kernels(self) -> str:
         t = self.launched_config
-        if t in (3, 4, 5, 6) and self.precision == 0:
-            return "pencil::k_prep + k_sweeps<z, y, x> + k_finish"
+        if self.swept:
+            if self.precision == 0:
+                return "pencil::k_prep + k_sweeps<z, y, x> + k_finish"
+            return ("pencil::k_prep + k_sweeps_mixed<z, y> + k_sweep_x_finish" if self.case.ns <= 2
+                    else "pencil::k_prep + k_sweeps_mixed<z, y, x> + k_finish")
         if t in (3, 4, 5, 6):
             yz = ("k_pencil_staged<z> + k_pencil_staged<y>" if t < 5 else
                   "k_pencil_staged<z, flow> + k_pencil_staged<z, species> + "

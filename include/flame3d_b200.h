@@ -373,9 +373,11 @@ int flame_rk_stage(const FlameGrid *g, flame_stream_t stream, int stage, double 
  * with one CTA per SM, 16x8x8 with two, 8x8x8 with two); 3 to 6 = sweeps along the grid axes that
  * need b->scratch.  FP64 runs 3 to 6 as the same three launches: a prep pass, the z, y and x
  * sweeps side by side, the finish (RK3 update, c2Prim, transport, ghosts); the interior of Q_out
- * and rhoi_out holds the x sweep's part between the last two.  In mixed precision 3 = four
- * barrier-free launches (a prep pass and z, y, x warp-per-pencil sweeps, the x sweep finishing
- * the stage); 4 = configuration 3 with the finish in a fifth, per-cell launch, bit-identical to 3;
+ * and rhoi_out holds the x sweep's part between the last two.  In mixed precision 3 and 4 run
+ * likewise (up to two species the x sweep is apart and finishes the stage; from three on the
+ * interior of trans_out is used in between as well); one species on at least 2^20 cells takes
+ * four barrier-free launches (a prep pass and z, y, x warp-per-pencil sweeps, the x sweep
+ * finishing the stage), with configuration 4 the finish in a fifth, bit-identical to 3;
  * 5, 6 = configurations 3, 4 with each z / y sweep split into a flow sweep and a species sweep
  * (fewer registers and shared-memory slots per sweep when there are many species).  The
  * autotuner picks the configuration per grid, species count and precision.  Transport law 2 runs

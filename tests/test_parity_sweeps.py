@@ -51,3 +51,27 @@ def test_sweeps_match_oracle(f3d, oracle, cuda_ok, nx, ny, nz, ns, law):
             scale = vel if 1 <= n <= 3 else np.linalg.norm(oc.Q[n].ravel())
             assert np.linalg.norm((Q[n] - oc.Q[n]).ravel()) <= 1e-12 * scale, (s, n)
         assert np.linalg.norm((r - oc.rhoi).ravel()) <= 1e-12 * np.linalg.norm(oc.rhoi.ravel()), s
+
+
+@pytest.mark.parametrize("nx,ny,nz,ns", [
+    (4, 4, 4, 1), (17, 27, 26, 2), (33, 9, 53, 3), (16, 12, 28, 4), (40, 30, 7, 7), (9, 26, 27, 8),
+    (251, 4, 5, 9),
+])
+def test_mixed_sweeps_match_the_staged_sweeps(f3d, cuda_ok, nx, ny, nz, ns):
+    """Mixed precision: the sweeps in one launch against the staged ones (which the persistent
+    batch runs) on the same case.  Both evaluate the same FP32 expressions, so a step agrees to
+    the last bit."""
+    import torch
+    case = _case(f3d, nx, ny, nz, ns, 1, seed=62)
+    S, B = f3d.solver_module(), f3d.batch_module()
+    one, ref = (S.DeviceCase(case, precision=1, tile=3) for _ in range(2))
+    batch = B.Batch([ref], mode="persistent")
+    assert one.swept
+    for _ in range(2):
+        one.step()
+        batch.step()
+    batch.status()
+    batch.close()
+    for a, b in ((one.U, ref.U), (one.Q[one.cur], ref.Q[ref.cur]), (one.rhoi[one.cur], ref.rhoi[ref.cur]),
+                 (one.T[one.cur], ref.T[ref.cur])):
+        assert torch.equal(a, b)
