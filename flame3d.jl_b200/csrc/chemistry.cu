@@ -411,8 +411,8 @@ __global__ void __launch_bounds__(128) k_eval_ns(Dims D, double *U, double *Q, d
     U[p + 4 * np] = u4 + dei;
     ein += dei;
     const MixPoly<NS> mp(th, r);
-    T = jmax(get_T_mix<NS>(mp, th, ein, r), kEps);
-    const double pr = jmax(p_mixture<NS>(th, NS, T, r), kEps);
+    T = jmax(get_T_mix<NS>(mp, th, ein), kEps);
+    const double pr = jmax(th.Ru * T * mp.wsum, kEps);
     Q[p + 4 * np] = pr;
     Q[p + 5 * np] = T;
     Q[p + 6 * np] = ein;

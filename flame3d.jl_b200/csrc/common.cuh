@@ -46,6 +46,33 @@ __device__ __forceinline__ int64_t tag_at(const int64_t *tag, long long p) {
     return tag ? tag[p] : 0;
 }
 
+// Reciprocal and reciprocal square root for the fused FP64 paths: the hardware's approximation
+// (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64) refined by Newton's iteration, without the
+// branches of the correctly rounded forms.  The seed is good to about 2^-20 and one step of third
+// order, x (1 + e + e^2) with e = 1 - d x, leaves it below 2^-57 before the rounding of the last
+// multiply-add.  Arguments are normal, positive or negative (rsqrt: positive); other arguments
+// give NaN or infinity.
+__device__ __forceinline__ double fast_rcp(double d) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    const double e = fma(-d, x, 1.0);
+    return fma(x, fma(e, e, e), x);
+}
+// a / b: the quotient by fast_rcp and one correction from its residual, which leaves it within
+// rounding of the correctly rounded one (no branch and no call, so a kernel near its register
+// limit does not spill around it).
+__device__ __forceinline__ double fast_div(double a, double b) {
+    const double r = fast_rcp(b), q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
+// x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2
+__device__ __forceinline__ double fast_rsqrt(double d) {
+    double x;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    const double e = fma(-d * x, x, 1.0);
+    return fma(x * e, fma(0.375, e, 0.5), x);
+}
+
 // ------------------------------------------------------------------ NASA-7 thermo (thermo.jl)
 // h_specs, thermo.jl:107-133 (J/kg)
 __device__ __forceinline__ double h_spec(const FlameThermo &th, int n, double T, double T2,
@@ -162,7 +189,7 @@ struct MixPoly {
         smin = smax = t.coeffs_sep[0];
 #pragma unroll
         for (int n = 0; n < NS; ++n) {
-            const double w = r[n] / t.mw[n];
+            const double w = fast_div(r[n], t.mw[n]);
             wsum += w;
             const double *L = t.coeffs_lo + 7 * n, *H = t.coeffs_hi + 7 * n;
             lo[0] += w * (L[0] - 1), hi[0] += w * (H[0] - 1);
@@ -188,19 +215,16 @@ struct MixPoly {
 };
 
 template <int NS>
-__device__ double get_T_mix(const MixPoly<NS> &M, const FlameThermo &th, double ein,
-                            const double *rhoi) {
+__device__ double get_T_mix(const MixPoly<NS> &M, const FlameThermo &th, double ein) {
     const double tol = 1e-3;
     const double tmin = th.min_temp, tmax = th.max_temp;
     const double emin = M.e(tmin), emax = M.e(tmax);
     if (ein < emin) return tmin - (emin - ein) / M.cv(tmin);
     if (ein > emax) return tmax - (emax - ein) / M.cv(tmax);
-    double As = 0;
-    for (int n = 0; n < NS; ++n) As += (th.coeffs_lo[7 * n] - 1) * th.Ru / th.mw[n] * rhoi[n];
-    double t1 = ein / As;
+    double t1 = ein * fast_rcp(M.lo[0] * th.Ru);  // Σ_n (a1_n - 1) Ru / W_n ρ_n is the mixture's own
     if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     for (int it = 0; it < 30; ++it) {
-        double dt = (ein - M.e(t1)) / M.cv(t1);
+        double dt = (ein - M.e(t1)) * fast_rcp(M.cv(t1));
         if (dt > 100.0)
             dt = 100.0;
         else if (dt < -100.0)
@@ -278,26 +302,6 @@ __device__ __forceinline__ T wenoz_minus(T V1, T V2, T V3, T V4, T V5) {
     const T s33 = tmp1 * (a * a) + q4 * (b * b);
     return wenoz_combine<T>(s11, s22, s33, 11 * V3 - 7 * V4 + 2 * V5, -V4 + 5 * V3 + 2 * V2,
                             2 * V3 + 5 * V2 - V1);
-}
-
-// Reciprocal and reciprocal square root for the fused FP64 paths: the hardware's approximation
-// (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64) refined by Newton's iteration, without the
-// branches of the correctly rounded forms.  The seed is good to about 2^-20 and one step of third
-// order, x (1 + e + e^2) with e = 1 - d x, leaves it below 2^-57 before the rounding of the last
-// multiply-add.  Arguments are normal, positive or negative (rsqrt: positive); other arguments
-// give NaN or infinity.
-__device__ __forceinline__ double fast_rcp(double d) {
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    const double e = fma(-d, x, 1.0);
-    return fma(x, fma(e, e, e), x);
-}
-// x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2
-__device__ __forceinline__ double fast_rsqrt(double d) {
-    double x;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    const double e = fma(-d * x, x, 1.0);
-    return fma(x * e, fma(0.375, e, 0.5), x);
 }
 
 // max that propagates NaN (Julia's) in the arithmetic type
@@ -621,6 +625,15 @@ __device__ __forceinline__ void mix_tables_fill(const FlameThermo &th, const Fla
     }
 }
 
+// Reciprocal and square root of the mixture rule: FP64 by fast_rcp and fast_rsqrt (arguments
+// are positive and normal), FP32 the correctly rounded ones.
+__device__ __forceinline__ double rule_rcp(double x) { return fast_rcp(x); }
+__device__ __forceinline__ float rule_rcp(float x) { return 1 / x; }
+__device__ __forceinline__ double rule_sqrt(double x) { return x * fast_rsqrt(x); }
+__device__ __forceinline__ float rule_sqrt(float x) { return sqrt(x); }
+__device__ __forceinline__ double rule_div(double a, double b) { return a * fast_rcp(b); }
+__device__ __forceinline__ float rule_div(float a, float b) { return a / b; }
+
 template <typename MT>
 __device__ __forceinline__ MT dot5t(MT l1, MT l2, MT l3, MT l4, const MT *p) {
     return p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3] + l4 * p[4];
@@ -638,7 +651,7 @@ __device__ __forceinline__ void mixture_properties_pairs(MT T, MT P, const MT *X
     for (int n = 0; n < NS; ++n) mui[n] = sqT * dot5t<MT>(lgT, lgT2, lgT3, lgT4, cond + 5 * n);
     MT sum1 = 0, sum2 = 0;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) sum1 += X[k] * mui[k], sum2 += X[k] / mui[k];
+    for (int k = 0; k < NS; ++k) sum1 += X[k] * mui[k], sum2 += rule_div(X[k], mui[k]);
     lam = MT(0.5) * (sum1 + 1 / sum2);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
@@ -648,14 +661,14 @@ __device__ __forceinline__ void mixture_properties_pairs(MT T, MT P, const MT *X
     }
     MT rmu[NS];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) rmu[n] = 1 / mui[n];
+    for (int n = 0; n < NS; ++n) rmu[n] = rule_rcp(mui[n]);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {  // Wilke: row[n] = Σ_l X[l] W[n][l]
 #pragma unroll
         for (int l = 0; l < n; ++l) {
             const int i = n * NS + l;
             const MT vr = mui[n] * rmu[l];  // μ_n / μ_l
-            const MT f1 = 1 + sqrt(vr * pw[NS * NS + i]);
+            const MT f1 = 1 + rule_sqrt(vr * pw[NS * NS + i]);
             const MT t = f1 * f1 * pw[2 * NS * NS + i];
             row[n] += X[l] * t;                                 // W[n][l]
             row[l] += X[n] * (t * (mui[l] * rmu[n]) * pw[i]);  // W[l][n] = t / (vr wr)
@@ -664,7 +677,7 @@ __device__ __forceinline__ void mixture_properties_pairs(MT T, MT P, const MT *X
     }
     mu = 0;
 #pragma unroll
-    for (int n = 0; n < NS; ++n) mu += X[n] * mui[n] / row[n];
+    for (int n = 0; n < NS; ++n) mu += rule_div(X[n] * mui[n], row[n]);
 #pragma unroll
     for (int n = 0; n < NS; ++n) row[n] = 0;  // now Σ_{m≠n} X[m] / Dbin[n][m]
 #pragma unroll
@@ -672,14 +685,14 @@ __device__ __forceinline__ void mixture_properties_pairs(MT T, MT P, const MT *X
 #pragma unroll
         for (int m = n + 1; m < NS; ++m) {
             const MT t = T * sqT * dot5t<MT>(lgT, lgT2, lgT3, lgT4, bin + 5 * (m + NS * n));
-            const MT rt = 1 / t;
+            const MT rt = rule_rcp(t);
             row[n] += X[m] * rt;
             row[m] += X[n] * rt;
         }
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
         const MT s = row[n] * P;
-        Dk[n] = (1 - X[n]) / (s + MT(kEps));
+        Dk[n] = rule_div(1 - X[n], s + MT(kEps));
     }
 }
 
@@ -691,14 +704,15 @@ __device__ __forceinline__ void mixture_point(const FlameThermo &th, const Flame
                                               const MixTables<NS, MT> &mt, double T, double P,
                                               double rho_raw, const double *r, double &mu,
                                               double &lam, double *Dk) {
-    const double rhoinv = 1 / jmax(rho_raw, kEps);
+    const double rhoinv = fast_rcp(jmax(rho_raw, kEps));
     double X[NS];
     double yow = 0;
 #pragma unroll
-    for (int n = 0; n < NS; ++n) X[n] = jmax(r[n] * rhoinv, 0.0), yow += X[n] / th.mw[n];
-    const double yowinv = 1 / yow;
+    for (int n = 0; n < NS; ++n)
+        X[n] = fast_div(jmax(r[n] * rhoinv, 0.0), th.mw[n]), yow += X[n];
+    const double yowinv = fast_rcp(yow);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) X[n] = X[n] / th.mw[n] * yowinv;
+    for (int n = 0; n < NS; ++n) X[n] *= yowinv;
     if constexpr (sizeof(MT) == 8) {
         mixture_properties_pairs<NS, double>(T, P, X, mt.pw, tr.poly, Dk, lam, mu);
     } else {

@@ -449,7 +449,7 @@ struct Tile {
             const double u = Uc[1] * rinv, v = Uc[2] * rinv, w = Uc[3] * rinv;
             const double ei = jmax(Uc[4] - 0.5 * rho * (u * u + v * v + w * w), kEps);
             const double Tn = jmax(NS < 4 ? get_T<NS>(A.th, NS, ei, r)
-                                           : get_T_mix<NS>(MixPoly<NS>(A.th, r), A.th, ei, r),
+                                           : get_T_mix<NS>(MixPoly<NS>(A.th, r), A.th, ei),
                                    kEps);
             const double p = jmax(p_mixture<NS>(A.th, NS, Tn, r), kEps);
             double mu, lam, D;

@@ -492,34 +492,35 @@ __device__ __forceinline__ void finish_cell(const Args<QT> &A, int g, int gx, in
     }
     // c2Prim, utils.jl:2-48
     const double rho = jmax(Uc[0], kEps);
-    const double rinv = 1 / rho;
+    const double rinv = fast_div(1.0, rho);
     double sr = 0.0;
 #pragma unroll
     for (int n = 0; n < NS; ++n) r[n] = jmax(r[n], 0.0), sr += r[n];
-    const double sc = rho / sr;
+    const double sc = fast_div(rho, sr);
 #pragma unroll
     for (int n = 0; n < NS; ++n) r[n] *= sc;
     const double u = Uc[1] * rinv, v = Uc[2] * rinv, w = Uc[3] * rinv;
     const double ei = jmax(Uc[4] - 0.5 * rho * (u * u + v * v + w * w), kEps);
     double mu, lam, D, Tn, p;
     double Dk[LAW2 ? NS : 1];
-    if constexpr (NS < 4) {  // few species: the per-species sums are as cheap
+    if constexpr (NS < 4 && sizeof(QT) == 4) {
+        // few species in mixed precision: the per-species sums, which need fewer registers than
+        // the mixture's polynomials inside the x sweep (64^3, one species: 309 against 314 us)
         Tn = jmax(get_T<NS>(A.th, NS, ei, r), kEps);
         p = jmax(p_mixture<NS>(A.th, NS, Tn, r), kEps);
         if constexpr (!LAW2) transport_point<NS>(A.th, A.tr, Tn, rho, r, mu, lam, D);
     } else {  // the mixture's own polynomials (MixPoly): one evaluation per Newton iteration
         const MixPoly<NS> M(A.th, r);
-        Tn = jmax(get_T_mix<NS>(M, A.th, ei, r), kEps);
-        p = jmax(p_mixture<NS>(A.th, NS, Tn, r), kEps);
+        Tn = jmax(get_T_mix<NS>(M, A.th, ei), kEps);
+        p = jmax(A.th.Ru * Tn * M.wsum, kEps);
         if constexpr (!LAW2) {
             if (A.tr.law == 0) {
                 mu = A.tr.mu_ref, lam = A.tr.lambda_ref, D = A.tr.D_ref;
             } else {  // transport_point with cp_mix = Σ_n w_n cp_n / ρ from the same polynomials
-                const double rh = jmax(rho, kEps);
-                const double cpm = (M.cv(Tn) + A.th.Ru * M.wsum) / rh;
-                mu = A.tr.mu_ref * pow(Tn / A.tr.T_ref, A.tr.exponent);
-                lam = cpm * mu / A.tr.Pr;
-                D = lam / (rh * cpm);
+                const double rcp = M.cv(Tn) + A.th.Ru * M.wsum;  // ρ cp
+                mu = A.tr.mu_ref * pow(fast_div(Tn, A.tr.T_ref), A.tr.exponent);
+                lam = fast_div(rcp * rinv * mu, A.tr.Pr);
+                D = fast_div(lam, rcp);
             }
         }
     }
@@ -656,8 +657,12 @@ __device__ __forceinline__ void finish_thread(const Args<QT> &A, const MixTables
     finish_cell<NS, QT, LAW2>(A, g, gx, gy, gz, rhs, mt);
 }
 
+// At most 128 registers from four species on (nine need 150: four blocks instead of three per SM).
+// Its divisions are fast_div's: the correctly rounded ones bring calls, around which a kernel at
+// its register limit spills (96^3, nine species: 164 -> 145 us; k_finish_mix 407 -> 237 us; HBM
+// traffic alone takes 102 us).
 template <int NS, typename QT, bool X3>
-__global__ void __launch_bounds__(128) k_finish(const __grid_constant__ Args<QT> A) {
+__global__ void __launch_bounds__(128, NS < 4 ? 6 : 4) k_finish(const __grid_constant__ Args<QT> A) {
     finish_thread<NS, QT, false, X3>(A, nullptr, blockIdx.x);
 }
 
