@@ -96,7 +96,7 @@ __device__ __forceinline__ double cp_spec(const FlameThermo &th, int n, double T
 }
 
 // ei_specs, thermo.jl:136-160 (dimensionless e/R)
-__device__ __forceinline__ double ei_spec(const FlameThermo &th, int n, double T, double T2,
+__host__ __device__ __forceinline__ double ei_spec(const FlameThermo &th, int n, double T, double T2,
                                           double T3, double T4, double T5) {
     const double *lo = th.coeffs_lo + 7 * n;
     if (T < th.coeffs_sep[n])
@@ -107,7 +107,7 @@ __device__ __forceinline__ double ei_spec(const FlameThermo &th, int n, double T
 
 // InternalEnergy, thermo.jl:219-228 (J/m^3)
 template <int NS>
-__device__ __forceinline__ double internal_energy(const FlameThermo &th, int ns, double T,
+__host__ __device__ __forceinline__ double internal_energy(const FlameThermo &th, int ns, double T,
                                                   const double *rhoi) {
     double T2 = 0.5 * T * T;
     double T3 = 2.0 / 3.0 * T2 * T;

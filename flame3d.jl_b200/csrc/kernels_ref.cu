@@ -426,79 +426,100 @@ __global__ void k_fill_periodic(Dims D, double *__restrict__ A, int nv, int peri
 }
 
 // ------------------------------------------------------------------ boundary.jl:1-176
-// The inflow state of fill_x / fill_z (boundary.jl:10-43, 89-122): every Yi and ρi zeroed, the
-// inflow's Y set, ρ = ρmixture(P, T, Y) (thermo.jl:29-35), ρi = Y ρ, e = InternalEnergy(T, ρi),
-// then Q and U.
-__device__ void set_inflow(const Dims &D, long long p, double *Q, double *U, double *rhoi,
-                           double *Yi, const FlameThermo &th, const FlameInflow &in) {
-    const int ns = D.ns;
-    const long long np = D.np;
-    for (int n = 0; n < ns; ++n) Yi[p + n * np] = 0.0, rhoi[p + n * np] = 0.0;
-    for (int n = 0; n < ns; ++n) Yi[p + n * np] = in.Y[n];
+// The fills touch a shell of NG + 1 planes at either end of an axis.  A thread takes one field of
+// one point of the shell (launched over the shell alone): over the whole grid with every field of
+// a point in one thread, the threads with work were a few of each warp, each with a chain of up
+// to 12 + 2 ns loads and stores behind one another, and the inflow's state was formed at every
+// point (96x50x42, five species: fill_x 17.5, fill_y 9.2, fill_z 9.8 us; a step with them
+// 705 -> 624 us).
+//
+// Fields of a point: 0..6 Q, 7..11 U, 12.. ρi (with Yi where the inflow sets it).
+
+// The inflow state of fill_x / fill_z (boundary.jl:10-43, 89-122) is the same at every point, so
+// the launch forms it once: Yi the inflow's Y, ρ = ρmixture(P, T, Y) (thermo.jl:29-35), ρi = Y ρ,
+// e = InternalEnergy(T, ρi), then Q and U.
+struct InflowPoint {
+    double f[12 + FLAME_MAX_NS];  // Q, U, ρi
+    double Y[FLAME_MAX_NS];
+};
+inline InflowPoint inflow_point(int ns, const FlameThermo &th, const FlameInflow &in) {
+    InflowPoint s{};
     double yow = 0;
-    for (int n = 0; n < ns; ++n) yow += Yi[p + n * np] / th.mw[n];
+    for (int n = 0; n < ns; ++n) yow += in.Y[n] / th.mw[n];
     const double rho = in.P / (th.Ru * in.T * yow);
-    double r[FLAME_MAX_NS];
-    for (int n = 0; n < ns; ++n) {
-        rhoi[p + n * np] = Yi[p + n * np] * rho;
-        r[n] = rhoi[p + n * np];
-    }
-    const double ei = internal_energy<0>(th, ns, in.T, r);
+    for (int n = 0; n < ns; ++n) s.Y[n] = in.Y[n], s.f[12 + n] = in.Y[n] * rho;
+    const double ei = internal_energy<0>(th, ns, in.T, s.f + 12);
     const double u = in.u, v = in.v, w = in.w;
-    const double q[7] = {rho, u, v, w, in.P, in.T, ei};
-    for (int n = 0; n < 7; ++n) Q[p + n * np] = q[n];
-    U[p] = rho;
-    U[p + np] = u * rho;
-    U[p + 2 * np] = v * rho;
-    U[p + 3 * np] = w * rho;
-    U[p + 4 * np] = ei + 0.5 * rho * (u * u + v * v + w * w);
+    const double q[12] = {rho, u,       v,       w,       in.P, in.T, ei,
+                          rho, u * rho, v * rho, w * rho, ei + 0.5 * rho * (u * u + v * v + w * w)};
+    for (int n = 0; n < 12; ++n) s.f[n] = q[n];
+    return s;
 }
 
-__device__ void copy_point(const Dims &D, long long dst, long long src, double *Q, double *U,
-                           double *rhoi) {
-    for (int n = 0; n < 7 && Q; ++n) Q[dst + n * D.np] = Q[src + n * D.np];
-    for (int n = 0; n < 5 && U; ++n) U[dst + n * D.np] = U[src + n * D.np];
-    for (int n = 0; n < D.ns && rhoi; ++n) rhoi[dst + n * D.np] = rhoi[src + n * D.np];
+__device__ __forceinline__ void set_inflow(const Dims &D, long long p, int f, double *Q, double *U,
+                                           double *rhoi, double *Yi, const InflowPoint &in) {
+    double *a = f < 7 ? Q + f * D.np : f < 12 ? U + (f - 7) * D.np : rhoi + (f - 12) * D.np;
+    a[p] = in.f[f];
+    if (f >= 12) Yi[p + (f - 12) * D.np] = in.Y[f - 12];
+}
+
+__device__ __forceinline__ void copy_field(const Dims &D, long long dst, long long src, int f,
+                                           double *Q, double *U, double *rhoi) {
+    double *a = f < 7 ? Q : f < 12 ? U : rhoi;
+    if (!a) return;
+    a += (f < 7 ? f : f < 12 ? f - 7 : f - 12) * D.np;
+    a[dst] = a[src];
+}
+
+// The shell's points of an axis with n cells (position c of 2 (NG + 1), low end first) and the
+// launch over `across` points of it.
+__device__ __forceinline__ long long shell_pos(int c, int n, int ng) {
+    return c <= ng ? c : n + c - 2;  // high end: n + ng - 1 + (c - ng - 1)
+}
+inline dim3 shell_grid(long long points, int fields) {
+    return dim3((unsigned)((points + 255) / 256), (unsigned)fields);
 }
 
 // fill_x, boundary.jl:1-52 (0-based: inflow i <= NG, outlet i >= nx+NG-1 from nx+NG-2)
-__global__ void k_fill_x(Dims D, double *Q, double *U, double *rhoi, double *Yi, FlameThermo th,
-                         FlameInflow in, int rank, int nprocs) {
-    long long i = blockIdx.x * (long long)BX + threadIdx.x;
-    long long j = blockIdx.y * (long long)BY + threadIdx.y;
-    long long k = blockIdx.z * (long long)BZ + threadIdx.z;
-    if (i >= D.tx || j >= D.ty || k >= D.tz) return;
-    const long long p = D.P(i, j, k);
-    if (rank == 0 && i <= D.ng) set_inflow(D, p, Q, U, rhoi, Yi, th, in);
-    if (rank == nprocs - 1 && i >= D.nx + D.ng - 1)
-        copy_point(D, p, D.P(D.nx + D.ng - 2, j, k), Q, U, rhoi);
+__global__ void __launch_bounds__(256) k_fill_x(Dims D, double *Q, double *U, double *rhoi,
+                                                double *Yi, const __grid_constant__ InflowPoint in,
+                                                int rank, int nprocs) {
+    const long long t = blockIdx.x * 256LL + threadIdx.x;
+    const int m = 2 * (D.ng + 1);
+    if (t >= m * D.ty * D.tz) return;
+    const int c = (int)(t % m);
+    const long long row = t / m * D.tx, p = row + shell_pos(c, D.nx, D.ng);
+    if (c <= D.ng) {
+        if (rank == 0) set_inflow(D, p, blockIdx.y, Q, U, rhoi, Yi, in);
+    } else if (rank == nprocs - 1) {
+        copy_field(D, p, row + D.nx + D.ng - 2, blockIdx.y, Q, U, rhoi);
+    }
 }
 
-// fill_y (boundary.jl:54-80) on Q, U and fill_y_s (139-158) on ρi: the same rule
-__global__ void k_fill_y(Dims D, double *Q, double *U, double *rhoi) {
-    long long i = blockIdx.x * (long long)BX + threadIdx.x;
-    long long j = blockIdx.y * (long long)BY + threadIdx.y;
-    long long k = blockIdx.z * (long long)BZ + threadIdx.z;
-    if (i >= D.tx || j >= D.ty || k >= D.tz) return;
-    if (j <= D.ng)
-        copy_point(D, D.P(i, j, k), D.P(i, D.ng + 1, k), Q, U, rhoi);
-    else if (j >= D.ny + D.ng - 1)
-        copy_point(D, D.P(i, j, k), D.P(i, D.ny + D.ng - 2, k), Q, U, rhoi);
+// fill_y (boundary.jl:54-80) on Q, U and fill_y_s (139-158) on ρi: the same rule (f0: first field)
+__global__ void __launch_bounds__(256) k_fill_y(Dims D, double *Q, double *U, double *rhoi, int f0) {
+    const long long t = blockIdx.x * 256LL + threadIdx.x;
+    const int m = 2 * (D.ng + 1);
+    if (t >= m * D.tx * D.tz) return;
+    const long long i = t % D.tx, k = t / (m * D.tx);
+    const int c = (int)(t / D.tx % m);
+    copy_field(D, D.P(i, shell_pos(c, D.ny, D.ng), k),
+               D.P(i, c <= D.ng ? D.ng + 1 : D.ny + D.ng - 2, k), f0 + blockIdx.y, Q, U, rhoi);
 }
 
 // fill_z (boundary.jl:82-137): inflow k <= NG, outlet k >= nz+NG-1 copies Q, U only;
-// fill_z_s (160-176) with Q = U = null: the outlet copy of ρi
-__global__ void k_fill_z(Dims D, double *Q, double *U, double *rhoi, double *Yi, FlameThermo th,
-                         FlameInflow in, int inflow) {
-    long long i = blockIdx.x * (long long)BX + threadIdx.x;
-    long long j = blockIdx.y * (long long)BY + threadIdx.y;
-    long long k = blockIdx.z * (long long)BZ + threadIdx.z;
-    if (i >= D.tx || j >= D.ty || k >= D.tz) return;
-    const long long p = D.P(i, j, k);
-    if (inflow && k <= D.ng)
-        set_inflow(D, p, Q, U, rhoi, Yi, th, in);
-    else if (k >= D.nz + D.ng - 1)
-        copy_point(D, p, D.P(i, j, D.nz + D.ng - 2), Q, U, inflow ? nullptr : rhoi);
+// fill_z_s (160-176), inflow 0: the outlet copy of ρi
+__global__ void __launch_bounds__(256) k_fill_z(Dims D, double *Q, double *U, double *rhoi,
+                                                double *Yi, const __grid_constant__ InflowPoint in,
+                                                int inflow, int f0) {
+    const long long t = blockIdx.x * 256LL + threadIdx.x;
+    const long long plane = D.tx * D.ty;
+    const int m = inflow ? 2 * (D.ng + 1) : D.ng + 1, f = f0 + blockIdx.y;
+    if (t >= m * plane) return;
+    const int c = (int)(t / plane) + (inflow ? 0 : D.ng + 1);
+    const long long at = t % plane, p = at + plane * shell_pos(c, D.nz, D.ng);
+    if (c <= D.ng) set_inflow(D, p, f, Q, U, rhoi, Yi, in);
+    else copy_field(D, p, at + plane * (D.nz + D.ng - 2), f, Q, U, inflow ? nullptr : rhoi);
 }
 
 // CFL rate of every interior cell, reduced to its maximum (see flame_cfl_max).  A non-negative
@@ -814,8 +835,8 @@ int flame_fill_x(const FlameGrid *g, flame_stream_t s, double *Q, double *U, dou
     if (!Q || !U || !rhoi || !Yi || !th || !in || nprocs < 1 || rank < 0 || rank >= nprocs)
         return flame_fail(FLAME_EINVAL, "flame_fill_x: NULL argument or bad rank/nprocs");
     const Dims D = make_dims(*g);
-    k_fill_x<<<grid_for(D.tx, D.ty, D.tz), kBlock, 0, s>>>(D, Q, U, rhoi, Yi, *th, *in, rank,
-                                                           nprocs);
+    k_fill_x<<<shell_grid(2 * (D.ng + 1) * D.ty * D.tz, 12 + D.ns), 256, 0, s>>>(
+        D, Q, U, rhoi, Yi, inflow_point(D.ns, *th, *in), rank, nprocs);
     return flame_check_launch("flame_fill_x");
 }
 
@@ -823,7 +844,7 @@ int flame_fill_y(const FlameGrid *g, flame_stream_t s, double *Q, double *U) {
     if (int e = check_fill_grid(g, "flame_fill_y")) return e;
     if (!Q || !U) return flame_fail(FLAME_EINVAL, "flame_fill_y: NULL argument");
     const Dims D = make_dims(*g);
-    k_fill_y<<<grid_for(D.tx, D.ty, D.tz), kBlock, 0, s>>>(D, Q, U, nullptr);
+    k_fill_y<<<shell_grid(2 * (D.ng + 1) * D.tx * D.tz, 12), 256, 0, s>>>(D, Q, U, nullptr, 0);
     return flame_check_launch("flame_fill_y");
 }
 
@@ -833,7 +854,8 @@ int flame_fill_z(const FlameGrid *g, flame_stream_t s, double *Q, double *U, dou
     if (!Q || !U || !rhoi || !Yi || !th || !in)
         return flame_fail(FLAME_EINVAL, "flame_fill_z: NULL argument");
     const Dims D = make_dims(*g);
-    k_fill_z<<<grid_for(D.tx, D.ty, D.tz), kBlock, 0, s>>>(D, Q, U, rhoi, Yi, *th, *in, 1);
+    k_fill_z<<<shell_grid(2 * (D.ng + 1) * D.tx * D.ty, 12 + D.ns), 256, 0, s>>>(
+        D, Q, U, rhoi, Yi, inflow_point(D.ns, *th, *in), 1, 0);
     return flame_check_launch("flame_fill_z");
 }
 
@@ -841,7 +863,8 @@ int flame_fill_y_s(const FlameGrid *g, flame_stream_t s, double *rhoi) {
     if (int e = check_fill_grid(g, "flame_fill_y_s")) return e;
     if (!rhoi) return flame_fail(FLAME_EINVAL, "flame_fill_y_s: NULL argument");
     const Dims D = make_dims(*g);
-    k_fill_y<<<grid_for(D.tx, D.ty, D.tz), kBlock, 0, s>>>(D, nullptr, nullptr, rhoi);
+    k_fill_y<<<shell_grid(2 * (D.ng + 1) * D.tx * D.tz, D.ns), 256, 0, s>>>(D, nullptr, nullptr,
+                                                                            rhoi, 12);
     return flame_check_launch("flame_fill_y_s");
 }
 
@@ -849,10 +872,8 @@ int flame_fill_z_s(const FlameGrid *g, flame_stream_t s, double *rhoi) {
     if (int e = check_fill_grid(g, "flame_fill_z_s")) return e;
     if (!rhoi) return flame_fail(FLAME_EINVAL, "flame_fill_z_s: NULL argument");
     const Dims D = make_dims(*g);
-    const FlameThermo th{};
-    const FlameInflow in{};
-    k_fill_z<<<grid_for(D.tx, D.ty, D.tz), kBlock, 0, s>>>(D, nullptr, nullptr, rhoi, nullptr,
-                                                           th, in, 0);
+    k_fill_z<<<shell_grid((D.ng + 1) * D.tx * D.ty, D.ns), 256, 0, s>>>(D, nullptr, nullptr, rhoi,
+                                                                        nullptr, InflowPoint{}, 0, 12);
     return flame_check_launch("flame_fill_z_s");
 }
 
