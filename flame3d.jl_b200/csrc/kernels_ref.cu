@@ -7,6 +7,8 @@
 // Launch shape: blocks of 32 x 4 x 2 threads with x fastest, so a warp reads 32 consecutive
 // FP64 values (256 B) of one SoA row instead of the reference's 4-wide x blocks (run.jl:66).
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace flame {
@@ -163,7 +165,12 @@ __device__ __forceinline__ double dtan4(const double *q, long long sn, long long
                   (1.0 / 12.0) * (q[2 * st] + q[-sn + 2 * st] - q[-2 * st] - q[-sn - 2 * st]));
 }
 
-__global__ void k_viscousFlux(Dims D, FaceGeom f, int d, double *__restrict__ Fv,
+// The direction (and below the species count, 0 for one known only at run time) is a compile-time
+// value, so that the arrays indexed by it stay in registers; the operations and their order are
+// the same.  128x64x64, one species: viscousFlux 42.6 -> 39.5 us a launch, specViscousFlux 29.9 ->
+// 19.7, c2Prim 66.5 -> 18.4, mixture 21.5 -> 14.9.
+template <int d>
+__global__ void k_viscousFlux(Dims D, FaceGeom f, double *__restrict__ Fv,
                               const double *__restrict__ Q, FlameMetrics m,
                               const double *__restrict__ lambda, const double *__restrict__ mu,
                               const double *__restrict__ Fh, const int64_t *__restrict__ tag) {
@@ -182,7 +189,7 @@ __global__ void k_viscousFlux(Dims D, FaceGeom f, int d, double *__restrict__ Fv
     const double Jac = (m.J[c - sn] + m.J[c]) * 0.5;
     const double mui = (mu[c - sn] + mu[c]) * 0.5;
     const double lami = (lambda[c - sn] + lambda[c]) * 0.5;
-    const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+    constexpr int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
     double gr[4][3];
     const int qv[4] = {1, 2, 3, 5};
 #pragma unroll
@@ -218,10 +225,11 @@ __global__ void k_viscousFlux(Dims D, FaceGeom f, int d, double *__restrict__ Fv
 }
 
 // ------------------------------------------------------------------- viscous.jl:430-665
-__global__ void k_specViscousFlux(Dims D, FaceGeom f, int d, double *__restrict__ Fd,
+template <int d, int NS>
+__global__ void k_specViscousFlux(Dims D, FaceGeom f, double *__restrict__ Fd,
                                   const double *__restrict__ Q, const double *__restrict__ Yi,
                                   FlameMetrics m, const double *__restrict__ Dk,
-                                  double *__restrict__ Fh, const FlameThermo th,
+                                  double *__restrict__ Fh, const __grid_constant__ FlameThermo th,
                                   const int64_t *__restrict__ tag) {
     long long fi = blockIdx.x * (long long)BX + threadIdx.x;
     long long fj = blockIdx.y * (long long)BY + threadIdx.y;
@@ -238,11 +246,14 @@ __global__ void k_specViscousFlux(Dims D, FaceGeom f, int d, double *__restrict_
     const double rho = (Q[c - sn] + Q[c]) * 0.5;
     const double T = (Q[c - sn + 5 * np] + Q[c + 5 * np]) * 0.5;
     const double T2 = 0.5 * T * T, T3 = 2.0 / 3.0 * T2 * T, T4 = T2 * T2, T5 = 0.8 * T4 * T;
-    const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
-    double Vk1[FLAME_MAX_NS], Vk2[FLAME_MAX_NS], Vk3[FLAME_MAX_NS];
+    constexpr int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+    constexpr int MAX = NS ? NS : FLAME_MAX_NS;
+    double Vk1[MAX], Vk2[MAX], Vk3[MAX];
     double sum1 = 0, sum2 = 0, sum3 = 0;
-    const int ns = D.ns;
-    for (int n = 0; n < ns; ++n) {
+    const int ns = NS ? NS : D.ns;
+#pragma unroll
+    for (int n = 0; n < MAX; ++n) {
+        if (n >= ns) break;
         const double *y = Yi + n * np + c;
         const double rhoDi = (Dk[c - sn + n * np] + Dk[c + n * np]) * rho;
         double dY[3];
@@ -258,7 +269,9 @@ __global__ void k_specViscousFlux(Dims D, FaceGeom f, int d, double *__restrict_
     const long long fo = fi + f.fx * (fj + f.fy * fk);
     const double *md = met + 3 * d;
     double fh1 = 0, fh2 = 0, fh3 = 0;
-    for (int n = 0; n < ns; ++n) {
+#pragma unroll
+    for (int n = 0; n < MAX; ++n) {
+        if (n >= ns) break;
         const double Yn = 0.5 * (Yi[c - sn + n * np] + Yi[c + n * np]);
         const double hn = h_spec(th, n, T, T2, T3, T4, T5);
         const double V1 = Vk1[n] - sum1 * Yn, V2 = Vk2[n] - sum2 * Yn, V3 = Vk3[n] - sum3 * Yn;
@@ -322,8 +335,9 @@ __global__ void k_linComb(Dims D, double *__restrict__ U, const double *__restri
 }
 
 // ------------------------------------------------------------------- utils.jl:2-48
+template <int NS>
 __global__ void k_c2Prim(Dims D, const double *__restrict__ U, double *__restrict__ Q,
-                         double *__restrict__ rhoi, const FlameThermo th,
+                         double *__restrict__ rhoi, const __grid_constant__ FlameThermo th,
                          const int64_t *__restrict__ tag) {
     long long i = blockIdx.x * (long long)BX + threadIdx.x;
     long long j = blockIdx.y * (long long)BY + threadIdx.y;
@@ -331,21 +345,28 @@ __global__ void k_c2Prim(Dims D, const double *__restrict__ U, double *__restric
     if (i >= D.nx || j >= D.ny || k >= D.nz) return;
     const long long c = D.P(i + D.ng, j + D.ng, k + D.ng), np = D.np;
     if (tag_at(tag, c) != 0) return;
-    const int ns = D.ns;
+    constexpr int MAX = NS ? NS : FLAME_MAX_NS;
+    const int ns = NS ? NS : D.ns;
     const double rho = jmax(U[c], kEps);
     const double rhoinv = 1 / rho;
-    double r[FLAME_MAX_NS];
+    double r[MAX];
     double sr = 0.0;
-    for (int n = 0; n < ns; ++n) {
+#pragma unroll
+    for (int n = 0; n < MAX; ++n) {
+        if (n >= ns) break;
         r[n] = jmax(rhoi[c + n * np], 0.0);
         sr += r[n];
     }
-    for (int n = 0; n < ns; ++n) r[n] *= rho / sr;
+#pragma unroll
+    for (int n = 0; n < MAX; ++n)
+        if (n < ns) r[n] *= rho / sr;
     const double u = U[c + np] * rhoinv, v = U[c + 2 * np] * rhoinv, w = U[c + 3 * np] * rhoinv;
     const double ei = jmax(U[c + 4 * np] - 0.5 * rho * (u * u + v * v + w * w), kEps);
-    const double T = jmax(get_T<0>(th, ns, ei, r), kEps);
-    const double p = jmax(p_mixture<0>(th, ns, T, r), kEps);
-    for (int n = 0; n < ns; ++n) rhoi[c + n * np] = r[n];
+    const double T = jmax(get_T<NS>(th, ns, ei, r), kEps);
+    const double p = jmax(p_mixture<NS>(th, ns, T, r), kEps);
+#pragma unroll
+    for (int n = 0; n < MAX; ++n)
+        if (n < ns) rhoi[c + n * np] = r[n];
     Q[c] = rho, Q[c + np] = u, Q[c + 2 * np] = v, Q[c + 3 * np] = w;
     Q[c + 4 * np] = p, Q[c + 5 * np] = T, Q[c + 6 * np] = ei;
 }
@@ -362,25 +383,30 @@ __global__ void k_prim2c(Dims D, double *__restrict__ U, const double *__restric
 }
 
 // ------------------------------------------------------------------- thermo.jl:371-403
+// LAW2: the mixture-averaged law, whose work arrays no other instance carries.
+template <int NS, bool LAW2>
 __global__ void k_mixture(Dims D, const double *__restrict__ Q, const double *__restrict__ rhoi,
                           double *__restrict__ Yi, double *__restrict__ lambda,
-                          double *__restrict__ mu, double *__restrict__ Dk, const FlameThermo th,
-                          const FlameTransport tr, const int64_t *__restrict__ tag) {
+                          double *__restrict__ mu, double *__restrict__ Dk,
+                          const __grid_constant__ FlameThermo th, const FlameTransport tr, const int64_t *__restrict__ tag) {
     long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= D.np) return;
     if (tag_at(tag, c) == 1) return;
     const long long np = D.np;
-    const int ns = D.ns;
+    constexpr int MAX = NS ? NS : FLAME_MAX_NS;
+    const int ns = NS ? NS : D.ns;
     const double T = Q[c + 5 * np];
     const double rho = jmax(Q[c], kEps);
     const double rhoinv = 1 / rho;
-    double Y[FLAME_MAX_NS];
-    for (int n = 0; n < ns; ++n) {
+    double Y[MAX];
+#pragma unroll
+    for (int n = 0; n < MAX; ++n) {
+        if (n >= ns) break;
         Y[n] = jmax(rhoi[c + n * np] * rhoinv, 0.0);
         Yi[c + n * np] = Y[n];
     }
     double mv, lv, dv;
-    if (tr.law == 2) {  // Y2X (thermo.jl:38-52), then mixtureProperties
+    if constexpr (LAW2) {  // Y2X (thermo.jl:38-52), then mixtureProperties
         double yow = 0;
         for (int n = 0; n < ns; ++n) yow += Y[n] / th.mw[n];
         const double yowinv = 1 / yow;
@@ -395,7 +421,9 @@ __global__ void k_mixture(Dims D, const double *__restrict__ Q, const double *__
     } else {
         const double T2 = T * T, T3 = T2 * T, T4 = T2 * T2;
         double cpm = 0;
-        for (int n = 0; n < ns; ++n) cpm += cp_spec(th, n, T, T2, T3, T4) * Y[n] / th.mw[n];
+#pragma unroll
+        for (int n = 0; n < MAX; ++n)
+            if (n < ns) cpm += cp_spec(th, n, T, T2, T3, T4) * Y[n] / th.mw[n];
         cpm *= th.Ru;
         mv = tr.mu_ref * pow(T / tr.T_ref, tr.exponent);
         lv = cpm * mv / tr.Pr;
@@ -622,6 +650,18 @@ __global__ void k_count_nonfinite(long long n, const double *__restrict__ A, uns
 
 using namespace flame;
 
+// Calls f with the species count as an integral_constant: 1 to 9, or 0 for a run-time count.
+template <typename F>
+static void by_species(int ns, const F &f) {
+    switch (ns) {
+#define CASE(N) \
+    case N: return f(std::integral_constant<int, N>());
+        CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9)
+#undef CASE
+        default: return f(std::integral_constant<int, 0>());
+    }
+}
+
 // ========================================================================= C ABI
 extern "C" {
 
@@ -700,8 +740,8 @@ static int visc_dir(const FlameGrid *g, flame_stream_t s, int d, double *Fv, con
         return flame_fail(FLAME_EINVAL, "%s: NULL array", name);
     Dims D = make_dims(*g);
     FaceGeom f = face_geom(D, d);
-    k_viscousFlux<<<grid_for(f.fx, f.fy, f.fz), kBlock, 0, s>>>(D, f, d, Fv, Q, m, lambda, mu,
-                                                                 Fh, tag);
+    const auto k = d == 0 ? k_viscousFlux<0> : d == 1 ? k_viscousFlux<1> : k_viscousFlux<2>;
+    k<<<grid_for(f.fx, f.fy, f.fz), kBlock, 0, s>>>(D, f, Fv, Q, m, lambda, mu, Fh, tag);
     return flame_check_launch(name);
 }
 int flame_viscousFlux_x(const FlameGrid *g, flame_stream_t s, double *Fv, const double *Q,
@@ -731,8 +771,12 @@ static int spec_dir(const FlameGrid *g, flame_stream_t s, int d, double *Fd, con
         return flame_fail(FLAME_EINVAL, "%s: NULL argument", name);
     Dims D = make_dims(*g);
     FaceGeom f = face_geom(D, d);
-    k_specViscousFlux<<<grid_for(f.fx, f.fy, f.fz), kBlock, 0, s>>>(D, f, d, Fd, Q, Yi, m, Dk,
-                                                                     Fh, *th, tag);
+    by_species(g->ns, [&](auto ns) {
+        constexpr int NS = decltype(ns)::value;
+        const auto k = d == 0 ? k_specViscousFlux<0, NS>
+                              : d == 1 ? k_specViscousFlux<1, NS> : k_specViscousFlux<2, NS>;
+        k<<<grid_for(f.fx, f.fy, f.fz), kBlock, 0, s>>>(D, f, Fd, Q, Yi, m, Dk, Fh, *th, tag);
+    });
     return flame_check_launch(name);
 }
 int flame_specViscousFlux_x(const FlameGrid *g, flame_stream_t s, double *Fd, const double *Q,
@@ -793,7 +837,10 @@ int flame_c2Prim(const FlameGrid *g, flame_stream_t s, const double *U, double *
     if (int e = flame_check_grid(g, "flame_c2Prim")) return e;
     if (!U || !Q || !rhoi || !th) return flame_fail(FLAME_EINVAL, "flame_c2Prim: NULL argument");
     Dims D = make_dims(*g);
-    k_c2Prim<<<grid_for(D.nx, D.ny, D.nz), kBlock, 0, s>>>(D, U, Q, rhoi, *th, tag);
+    by_species(g->ns, [&](auto ns) {
+        k_c2Prim<decltype(ns)::value>
+            <<<grid_for(D.nx, D.ny, D.nz), kBlock, 0, s>>>(D, U, Q, rhoi, *th, tag);
+    });
     return flame_check_launch("flame_c2Prim");
 }
 
@@ -816,8 +863,15 @@ int flame_mixture(const FlameGrid *g, flame_stream_t s, const double *Q, const d
     if (tr->law == 2 && !tr->poly)
         return flame_fail(FLAME_EINVAL, "flame_mixture: law 2 needs the polynomial fits (poly)");
     Dims D = make_dims(*g);
-    k_mixture<<<(unsigned)((D.np + 255) / 256), 256, 0, s>>>(D, Q, rhoi, Yi, lambda, mu, Dk, *th,
-                                                              *tr, tag);
+    const unsigned blocks = (unsigned)((D.np + 255) / 256);
+    if (tr->law == 2) {
+        k_mixture<0, true><<<blocks, 256, 0, s>>>(D, Q, rhoi, Yi, lambda, mu, Dk, *th, *tr, tag);
+    } else {
+        by_species(g->ns, [&](auto ns) {
+            k_mixture<decltype(ns)::value, false>
+                <<<blocks, 256, 0, s>>>(D, Q, rhoi, Yi, lambda, mu, Dk, *th, *tr, tag);
+        });
+    }
     return flame_check_launch("flame_mixture");
 }
 
