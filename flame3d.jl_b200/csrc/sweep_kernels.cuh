@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(SweepSlots<NS, MIXD>::NT, SweepSlots<NS, MIXD>
     k_sweeps(const __grid_constant__ Args<double> A, const __grid_constant__ SweepShape P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *S = reinterpret_cast<double *>(smem_raw);
+    chain_begin();
     const int b = blockIdx.x;
     if (b < P.y0) sweep_block<2, NS, MIXD>(A, P, b, S);
     else if (b < P.x0) sweep_block<1, NS, MIXD>(A, P, b - P.y0, S);
@@ -615,7 +616,8 @@ inline SweepShape sweep_shape(int nx, int ny, int nz) {
     }
     const long long all = ny * (long long)nz;
     double best = 1e300;
-    for (int nseg = 1; nseg <= (nx + 25) / 26 + 1; ++nseg) {
+    const int fewest = (nx + NT - 7) / (NT - 6);  // cuts with which a row fits a block
+    for (int nseg = fewest; nseg <= fewest + 24 && nseg <= (nx + 25) / 26 + 1; ++nseg) {
         const int own = (nx + nseg - 1) / nseg;
         for (int rows = 1; rows * (own + 6) <= NT; ++rows) {
             const double warps = (rows * (own + 6) + 31) / 32 + (rows * (own + 1) + 31) / 32;
