@@ -9,7 +9,7 @@ one-launch-per-stage kernel.  A "step" is one SSP-RK3 step (three stages).
   e2e    the same metric through the public host-buffer call (DeviceCase.advance_from_host):
          every step uploads the ghosted Q and rho_i from pinned memory and downloads them
   roofline  one RK3 stage (the unit the algorithmic bytes are defined for: one fused launch in
-         configurations 0-2, the prep pass and three pencil sweeps in configuration 3) against
+         configurations 0-2, the prep pass, the sweeps and the finish in configuration 3) against
          the measured HBM copy bandwidth, with B_alg = 8 (41 + 3 Ns + [Ns >= 2] Ns) bytes per
          interior cell-stage; `traffic` is the DRAM bytes per stage from an ncu capture
   cpu_baseline  the oracle (C++ FP64 restatement, OpenMP over all host cores) on a bounded
@@ -806,8 +806,8 @@ def main() -> int:
                         "flop_per_cell_stage": fc["flop_per_cell_stage"],
                         "peak_source": "measured (csrc/probe/fp64_peak.cu, this run)",
                         "counts_source": counts.get("source")}
-        roof["limiter"] = ("neither roof: FP64 issue and latency at 24 of 64 warps per SM on "
-                           "the y and z sweeps (profiles/pencil_stage_traffic_jet128x64x64.md)")
+        roof["limiter"] = ("neither roof: latency and barriers at 24 of 64 warps per SM in the "
+                           "sweeps (profiles/sweeps_jet128x64x64_fp64.md)")
 
     cpu = None
     if not args.no_cpu:

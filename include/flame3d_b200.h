@@ -17,7 +17,7 @@
  *   - Global state of the library: a per-thread error string; per device, atomic flags
  *     recording that a kernel's dynamic shared-memory limit has been raised (set once, never
  *     cleared; host threads on different streams may call concurrently); the
- *     persistent batch's constant-memory descriptor table (one per device, see flame_batch_*);
+ *     persistent batch's constant-memory descriptor tables (per device, see flame_batch_*);
  *     and, used only by flame_rk_stage_noalloc, a library-held scratch array with its
  *     per-device address cache (described at that entry point).  No call allocates device
  *     memory.
@@ -434,14 +434,16 @@ int flame_transport_boundary(const FlameGrid *g, flame_stream_t stream, const vo
  * together by persistent kernels.  Cases are grouped by species count and transport family
  * (laws 0 and 1, or law 2) and cut into chunks of at most 20; per chunk and stage the chunk's
  * descriptors go into a constant-memory table and the persistent kernels run one after the
- * other on the stream, each over its part of a (case, block) work list.  Laws 0 and 1 take
+ * other on the stream, each over its part of a (case, block) work list.  Up to 2^22 cells in all,
+ * chunks of different species counts run side by side on streams the batch owns, forked from the
+ * caller's stream and joined back to it within each flame_batch_stage.  Laws 0 and 1 take
  * configuration 3's shape, two kernels: the prep, z-sweep and y-sweep blocks of every case of
  * the chunk in list order, a case's sweep blocks waiting on a device counter for that case's
  * prep blocks; then the x-sweep blocks, which finish the stage.  Law 2 takes configuration 6's
  * shape, four: prep and flow-only sweeps (with the same waits), the species sweeps, the x
  * sweeps, and the finish with the mixture rule.  Every wait is bounded: when one runs out
  * (about half a second) the batch's error word is set and the remaining items are skipped;
- * flame_batch_status reports it.  The constant table is one per device: persistent batches on
+ * flame_batch_status reports it.  The constant tables are per device: persistent batches on
  * one device must not run concurrently.  Descriptors and work lists for all stages and both
  * in/out parities go once into caller-owned device workspace, so a captured CUDA graph of
  * flame_batch_stage calls replays without host work.  parity 0 advances buf.*_in -> buf.*_out,
