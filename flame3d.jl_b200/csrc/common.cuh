@@ -470,7 +470,11 @@ __device__ __forceinline__ double split_fast(double rho, double u, double v, dou
     return E1;
 }
 
-// FP32: the reference's form with its divisions folded into two reciprocals and an rsqrt.
+// FP32: the reference's form with its divisions folded into two reciprocals and an rsqrt.  The
+// outputs are STRIDE apart, so that a caller can have them stored where it stages them: through
+// two arrays the compiler held all ten to the end and stored them together, and a mixed step of
+// the 256x128x128 jet took 4328 us, with each stored as it is formed 4286.
+template <int STRIDE = 1>
 __device__ __forceinline__ float split_fast(float rho, float u, float v, float w, float p,
                                             float ei, float A1, float A2, float A3, float *fp,
                                             float *fm) {
@@ -497,15 +501,15 @@ __device__ __forceinline__ float split_fast(float rho, float u, float v, float w
     const float tmp1 = h * rho * (rho * gm1 * inv);                  // ρ/(2γ)
     const float tmp2 = 2 * gm1;
     fp[0] = tmp1 * (tmp2 * E1P + E2P + E3P);
-    fp[1] = tmp1 * (tmp2 * E1P * u + E2P * uc1 + E3P * uc2);
-    fp[2] = tmp1 * (tmp2 * E1P * v + E2P * vc1 + E3P * vc2);
-    fp[3] = tmp1 * (tmp2 * E1P * w + E2P * wc1 + E3P * wc2);
-    fp[4] = tmp1 * (E1P * vv + E2P * vvc1 + E3P * vvc2 + W2 * (E2P + E3P));
+    fp[STRIDE] = tmp1 * (tmp2 * E1P * u + E2P * uc1 + E3P * uc2);
+    fp[2 * STRIDE] = tmp1 * (tmp2 * E1P * v + E2P * vc1 + E3P * vc2);
+    fp[3 * STRIDE] = tmp1 * (tmp2 * E1P * w + E2P * wc1 + E3P * wc2);
+    fp[4 * STRIDE] = tmp1 * (E1P * vv + E2P * vvc1 + E3P * vvc2 + W2 * (E2P + E3P));
     fm[0] = tmp1 * (tmp2 * E1M + E2M + E3M);
-    fm[1] = tmp1 * (tmp2 * E1M * u + E2M * uc1 + E3M * uc2);
-    fm[2] = tmp1 * (tmp2 * E1M * v + E2M * vc1 + E3M * vc2);
-    fm[3] = tmp1 * (tmp2 * E1M * w + E2M * wc1 + E3M * wc2);
-    fm[4] = tmp1 * (E1M * vv + E2M * vvc1 + E3M * vvc2 + W2 * (E2M + E3M));
+    fm[STRIDE] = tmp1 * (tmp2 * E1M * u + E2M * uc1 + E3M * uc2);
+    fm[2 * STRIDE] = tmp1 * (tmp2 * E1M * v + E2M * vc1 + E3M * vc2);
+    fm[3 * STRIDE] = tmp1 * (tmp2 * E1M * w + E2M * wc1 + E3M * wc2);
+    fm[4 * STRIDE] = tmp1 * (E1M * vv + E2M * vvc1 + E3M * vvc2 + W2 * (E2M + E3M));
     return E1;
 }
 

@@ -243,10 +243,15 @@ __device__ __forceinline__ void point_phase(const Args<QT> &A, CT *S, int l, int
     const CT A1 = mv[3 * DIR], A2 = mv[3 * DIR + 1], A3 = mv[3 * DIR + 2];
     // Steger-Warming split, split.jl:17-89
     {
-        CT fp[5], fm[5];
-        const CT E1 = split_fast(rho, u, v, w, p, ei, A1, A2, A3, fp, fm);
+        CT E1;
+        if constexpr (sizeof(CT) == 4) {
+            E1 = split_fast<32>(rho, u, v, w, p, ei, A1, A2, A3, &SV(0), &SV(5));
+        } else {
+            CT fp[5], fm[5];
+            E1 = split_fast(rho, u, v, w, p, ei, A1, A2, A3, fp, fm);
 #pragma unroll
-        for (int n = 0; n < 5; ++n) SV(n) = fp[n], SV(5 + n) = fm[n];
+            for (int n = 0; n < 5; ++n) SV(n) = fp[n], SV(5 + n) = fm[n];
+        }
         // species, split.jl:101-130
         const CT Ep = h * (E1 + fabs(E1)), Em = h * (E1 - fabs(E1));
 #pragma unroll
