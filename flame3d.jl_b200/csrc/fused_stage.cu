@@ -126,12 +126,12 @@ int transport_ns(int ns, int np, cudaStream_t s, const void *Q, const double *ri
 }  // namespace flame
 
 namespace {
-// Every array of the stage must hold fewer than 2^31 elements (32-bit indices).  Extents are
-// widened to 64 bits and multiplied one at a time, so absurd extents cannot wrap into a small
-// product: before each multiplication the partial product is below 2^28 and the factor below
-// 2^32.
-int check_sizes(const FlameGrid *g, const char *what) {
-    const long long nv = g->ns > 10 ? g->ns : 10;
+// Every array of the call must hold fewer than 2^31 elements (32-bit indices): `fields` is what
+// the widest of them holds, at least the ten metric fields.  Extents are widened to 64 bits and
+// multiplied one at a time, so absurd extents cannot wrap into a small product: before each
+// multiplication the partial product is below 2^28 and the factor below 2^32.
+int check_sizes(const FlameGrid *g, int fields, const char *what) {
+    const long long nv = fields > 10 ? fields : 10;
     const long long ext[3] = {(long long)g->nx + 2LL * g->ng, (long long)g->ny + 2LL * g->ng,
                               (long long)g->nz + 2LL * g->ng};
     long long np = 1;
@@ -151,7 +151,8 @@ static int transport_call(const FlameGrid *g, flame_stream_t s, const void *Q,
                           const FlameTransport *tr, int precision, bool shell,
                           const char *what) {
     if (int e = flame_check_grid(g, what)) return e;
-    if (int e = check_sizes(g, what)) return e;
+    // law 2 stores 2 + ns transport fields
+    if (int e = check_sizes(g, tr && tr->law == 2 ? 2 + g->ns : g->ns, what)) return e;
     if (!Q || !rhoi || !trans || !th || !tr) return flame_fail(FLAME_EINVAL, "%s: NULL argument", what);
     if (tr->law < 0 || tr->law > 2)
         return flame_fail(FLAME_EINVAL, "%s: transport law %d unknown", what, tr->law);
@@ -188,7 +189,8 @@ extern "C" int flame_rk_stage_tiled(const FlameGrid *g, flame_stream_t s, int st
     static const char *kNames[3] = {"flame_rk_stage 1", "flame_rk_stage 2", "flame_rk_stage 3"};
     flame::NvtxRange range(kNames[(stage >= 1 && stage <= 3) ? stage - 1 : 0]);
     if (int e = flame_check_grid(g, "flame_rk_stage")) return e;
-    if (int e = check_sizes(g, "flame_rk_stage")) return e;
+    // the right-hand sides of the pencil configurations hold 5 + ns fields
+    if (int e = check_sizes(g, tile >= 3 ? 5 + g->ns : g->ns, "flame_rk_stage")) return e;
     if (!b || !m || !th || !tr || !b->U || !b->Un || !b->Q_in || !b->Q_out || !b->rhoi_in ||
         !b->rhoi_out || !b->rhon || !b->trans_in || !b->trans_out || !m->J || !m->dxidx ||
         !m->dxidy || !m->dxidz || !m->detadx || !m->detady || !m->detadz || !m->dzetadx ||

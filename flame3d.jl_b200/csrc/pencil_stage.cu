@@ -236,8 +236,10 @@ int check_case(const FlameCaseDesc &c, int i) {
         return flame_fail(FLAME_EINVAL, "flame_batch: case %d extents must be >= %d", i, FLAME_NG);
     const long long np =
         ((long long)c.grid.nx + 8) * ((long long)c.grid.ny + 8) * ((long long)c.grid.nz + 8);
+    // 32-bit indices: the widest arrays are the ten metric fields and the right-hand sides
+    const int fields = std::max(10, 5 + c.grid.ns);
     if (c.grid.nx > (1 << 20) || c.grid.ny > (1 << 20) || c.grid.nz > (1 << 20) ||
-        np * 10 >= (1LL << 31))
+        np * fields >= (1LL << 31))
         return flame_fail(FLAME_EINVAL, "flame_batch: case %d too large", i);
     const FlameStageBuffers &b = c.buf;
     if (!b.U || !b.Un || !b.Q_in || !b.Q_out || !b.rhoi_in || !b.rhoi_out || !b.rhon ||

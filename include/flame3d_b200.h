@@ -383,7 +383,9 @@ int flame_rk_stage(const FlameGrid *g, flame_stream_t stream, int stage, double 
  * autotuner picks the configuration per grid, species count and precision.  Transport law 2 runs
  * on configurations 3-6, in mixed precision always with configuration 6's launches (its species
  * sweeps and x sweep read each species' D_k, and the finish evaluates the mixture rule per cell);
- * configurations 0-2 refuse it with FLAME_EUNSUPPORTED. */
+ * configurations 0-2 refuse it with FLAME_EUNSUPPORTED.  Indices are 32-bit: a grid of which an
+ * array would reach 2^31 elements (ten metric fields; 5 + ns right-hand sides with configurations
+ * 3 to 6) is refused with FLAME_EINVAL. */
 int flame_rk_stage_tiled(const FlameGrid *g, flame_stream_t stream, int stage, double dt,
                          const FlameStageBuffers *b, const FlameMetrics *m,
                          const FlameThermo *thermo, const FlameTransport *transport,
