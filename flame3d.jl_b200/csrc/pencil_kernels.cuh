@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "sweep_shape.cuh"
 
 namespace flame {
 namespace pencil {

@@ -43,12 +43,6 @@ struct SweepSlots {
     static_assert(N <= MOST && MINB * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
 };
 
-// How the launch is cut: own cells per line and direction, lines per x block, threads per
-// block, and the first block of the y and of the x sweep (blocks [0, y0) are the z sweep's).
-struct SweepShape {
-    int own[3], rows, threads, y0, x0, blocks;
-};
-
 // Where the x sweep leaves field n of a cell for the finish: the stage's output arrays, whose
 // interior the finish of the same cell writes after it has read this (rhoi_out one value of 8
 // bytes per species; for the five flow fields Q_out's seven).
@@ -599,40 +593,6 @@ __global__ void __launch_bounds__(MixedSlots<NS>::NT, MixedSlots<NS>::MINB)
     k_sweep_x_finish(const __grid_constant__ Args<float> A, const __grid_constant__ SweepShape P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     mixed_block<0, NS, true>(A, P, blockIdx.x, reinterpret_cast<float *>(smem_raw));
-}
-
-// Cuts a launch.  y and z: C columns of n / nseg cells, at most 26 (the points of a block are
-// C (own + 6) <= 32 C).  x: the rows per block and the cut of a row that need the fewest warps
-// (those of the points and those of the faces) per cell.
-template <typename SL>
-inline SweepShape sweep_shape(int nx, int ny, int nz) {
-    constexpr int C = SL::C, NT = SL::NT;
-    SweepShape P{};
-    const int most = NT / C - 6;
-    const int ext[3] = {nx, ny, nz};
-    for (int d = 1; d < 3; ++d) {
-        const int nseg = (ext[d] + most - 1) / most;
-        P.own[d] = (ext[d] + nseg - 1) / nseg;
-    }
-    const long long all = ny * (long long)nz;
-    double best = 1e300;
-    const int fewest = (nx + NT - 7) / (NT - 6);  // cuts with which a row fits a block
-    for (int nseg = fewest; nseg <= fewest + 24 && nseg <= (nx + 25) / 26 + 1; ++nseg) {
-        const int own = (nx + nseg - 1) / nseg;
-        for (int rows = 1; rows * (own + 6) <= NT; ++rows) {
-            const double warps = (rows * (own + 6) + 31) / 32 + (rows * (own + 1) + 31) / 32;
-            const double blocks = double((all + rows - 1) / rows) * ((nx + own - 1) / own);
-            if (warps * blocks < best) best = warps * blocks, P.own[0] = own, P.rows = rows;
-        }
-    }
-    const int nxb = (nx + C - 1) / C;
-    P.y0 = nxb * ny * ((nz + P.own[2] - 1) / P.own[2]);
-    P.x0 = P.y0 + nxb * nz * ((ny + P.own[1] - 1) / P.own[1]);
-    P.blocks = P.x0 + (int)((all + P.rows - 1) / P.rows) * ((nx + P.own[0] - 1) / P.own[0]);
-    int t = P.rows * (P.own[0] + 6);
-    for (int d = 1; d < 3; ++d) t = t > C * (P.own[d] + 6) ? t : C * (P.own[d] + 6);
-    P.threads = (t + 31) / 32 * 32;
-    return P;
 }
 
 // Mixed precision: one species on at least 2^20 cells runs the staged sweeps (figures above).
