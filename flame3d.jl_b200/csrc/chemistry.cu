@@ -356,16 +356,27 @@ __global__ void __launch_bounds__(128) k_eval_ns(Dims D, double *U, double *Q, d
                                                  Mech M, const int64_t *tag, double Tcrit,
                                                  int transposed) {
     __shared__ MechTables<NS> t;
-    fill_tables<NS>(t, M, th);
-    __syncthreads();
     const long long c = blockIdx.x * 128LL + threadIdx.x;
     const long long ncell = (long long)D.nx * D.ny * D.nz;
-    if (c >= ncell) return;
-    const long long x = c % D.nx, y = (c / D.nx) % D.ny, z = c / ((long long)D.nx * D.ny);
+    long long x, y, z;
+    if (ncell < 1LL << 31) {  // 32-bit divisions where the cells allow
+        const unsigned q = (unsigned)c / (unsigned)D.nx;
+        x = (unsigned)c % (unsigned)D.nx, y = q % (unsigned)D.ny, z = q / (unsigned)D.ny;
+    } else {
+        x = c % D.nx, y = (c / D.nx) % D.ny, z = c / ((long long)D.nx * D.ny);
+    }
     const long long p = D.P(x + D.ng, y + D.ng, z + D.ng), np = D.np;
-    if (tag && tag[p] != 0) return;
-    double T = Q[p + 5 * np];
-    if (!(T > Tcrit)) return;
+    double T = 0.0;
+    bool hot = c < ncell && !(tag && tag[p] != 0);
+    if (hot) T = Q[p + 5 * np], hot = T > Tcrit;
+    // A block without a hot cell leaves the mechanism alone.  Eight species, 96^3 cells, explicit /
+    // point-implicit: no cell hot 25 / 33 -> 13 / 19 us (the run-time kernel, with fewer registers,
+    // 15 / 15), one cell in a hundred 110 / 205 -> 87 / 181, all of them 310 / 640 -> 296 / 635.  A
+    // loop over chunks in as many blocks as the GPU holds spills (all hot 352 / 691).
+    if (!__syncthreads_or(hot)) return;
+    fill_tables<NS>(t, M, th);
+    __syncthreads();
+    if (!hot) return;
     double sc[NS], w[NS], r[NS];
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
