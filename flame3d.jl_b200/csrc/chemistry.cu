@@ -233,13 +233,20 @@ __device__ __forceinline__ void fill_tables(MechTables<NS> &t, const Mech &M,
             const long long vf = M.vf[m + NS * n], vr = M.vr[m + NS * n];
             t.vf[n][m] = vf, t.vr[n][m] = vr;
             t.nu[n][m] = double(vr - vf);
-            t.ef[n][m] = M.ef[m + NS * n];
             fm |= (vf != 0 ? 1u : 0u) << m, rm |= (vr != 0 ? 1u : 0u) << m;
         }
         t.fmask[n] = fm, t.rmask[n] = rm;
-        t.type[n] = (int)M.type[n], t.sgm[n] = M.sgm[n];
-        for (int a = 0; a < 3; ++a) t.Arr[n][a] = M.Arr[3 * n + a], t.loP[n][a] = M.loP[3 * n + a];
-        for (int a = 0; a < 4; ++a) t.Troe[n][a] = M.Troe[4 * n + a];
+        const int type = (int)M.type[n];
+        t.type[n] = type, t.sgm[n] = M.sgm[n];
+        for (int a = 0; a < 3; ++a) t.Arr[n][a] = M.Arr[3 * n + a];
+        // only what the reaction's type uses is read, so the arrays may end with the last reaction
+        // that needs them
+        if (type == 2 || type == 3)
+            for (int m = 0; m < NS; ++m) t.ef[n][m] = M.ef[m + NS * n];
+        if (type == 3) {
+            for (int a = 0; a < 3; ++a) t.loP[n][a] = M.loP[3 * n + a];
+            for (int a = 0; a < 4; ++a) t.Troe[n][a] = M.Troe[4 * n + a];
+        }
     }
     if (threadIdx.x < NS) t.rmw[threadIdx.x] = 1 / th.mw[threadIdx.x];
 }
