@@ -47,23 +47,39 @@ __device__ __forceinline__ int64_t tag_at(const int64_t *tag, long long p) {
 }
 
 // Reciprocal and reciprocal square root for the fused FP64 paths: the hardware's approximation
-// (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64) refined by Newton's iteration, without the
-// branches of the correctly rounded forms.  The seed is good to about 2^-20 and one step of third
-// order, x (1 + e + e^2) with e = 1 - d x, leaves it below 2^-57 before the rounding of the last
-// multiply-add.  Arguments are normal, positive or negative (rsqrt: positive); other arguments
-// give NaN or infinity.
+// (PTX rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64) refined by one step of third order, without the
+// branches of the correctly rounded forms.  With e = 1 - d x the reciprocal is x / (1 - e), and
+// Householder's method (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
+// 1970) cuts the series after x (1 + e + e^2): a seed good to 2^-20 gives 2^-57 before rounding.
+// fast_rcp and fast_rsqrt are for the sweeps, whose arguments are normal (rsqrt: positive) with a
+// normal result: for zero and infinity they give NaN, and a reciprocal below the normal range is
+// flushed to zero.
 __device__ __forceinline__ double fast_rcp(double d) {
     double x;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
     const double e = fma(-d, x, 1.0);
     return fma(x, fma(e, e, e), x);
 }
-// a / b: the quotient by fast_rcp and one correction from its residual, which leaves it within
-// rounding of the correctly rounded one (no branch and no call, so a kernel near its register
-// limit does not spill around it).
+// The same where a zero or an infinity can occur: the seed is exact there, and the step that is
+// then NaN is left out.
+__device__ __forceinline__ double full_rcp(double d) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    const double e = fma(-d, x, 1.0), r = fma(x, fma(e, e, e), x);
+    return r == r ? r : x;
+}
+// a / b: the quotient by the refined reciprocal and one correction from its residual (P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, 1990), which leaves it
+// within rounding of the correctly rounded one (no branch and no call, so a kernel near its register
+// limit does not spill around it).  A zero or infinite operand, or a quotient that overflows, gives
+// what a division gives, by the seed; a quotient or reciprocal below the normal range may come out
+// as zero.
 __device__ __forceinline__ double fast_div(double a, double b) {
-    const double r = fast_rcp(b), q = a * r;
-    return fma(fma(-b, q, a), r, q);
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
+    const double e = fma(-b, x, 1.0), r = fma(x, fma(e, e, e), x), q = a * r;
+    const double c = fma(fma(-b, q, a), r, q);
+    return c == c ? c : a * x;
 }
 // x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2
 __device__ __forceinline__ double fast_rsqrt(double d) {
@@ -221,10 +237,10 @@ __device__ double get_T_mix(const MixPoly<NS> &M, const FlameThermo &th, double 
     const double emin = M.e(tmin), emax = M.e(tmax);
     if (ein < emin) return tmin - (emin - ein) / M.cv(tmin);
     if (ein > emax) return tmax - (emax - ein) / M.cv(tmax);
-    double t1 = ein * fast_rcp(M.lo[0] * th.Ru);  // Σ_n (a1_n - 1) Ru / W_n ρ_n is the mixture's own
+    double t1 = ein * full_rcp(M.lo[0] * th.Ru);  // Σ_n (a1_n - 1) Ru / W_n ρ_n is the mixture's own
     if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     for (int it = 0; it < 30; ++it) {
-        double dt = (ein - M.e(t1)) * fast_rcp(M.cv(t1));
+        double dt = (ein - M.e(t1)) * full_rcp(M.cv(t1));
         if (dt > 100.0)
             dt = 100.0;
         else if (dt < -100.0)
