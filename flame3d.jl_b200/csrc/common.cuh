@@ -645,13 +645,17 @@ __device__ __forceinline__ void mix_tables_fill(const FlameThermo &th, const Fla
     }
 }
 
-// Reciprocal and square root of the mixture rule: FP64 by fast_rcp and fast_rsqrt (arguments
-// are positive and normal), FP32 the correctly rounded ones.
-__device__ __forceinline__ double rule_rcp(double x) { return fast_rcp(x); }
+// Reciprocal, square root and quotient of the mixture rule: FP64 by the refined forms, with what
+// the exact operations give for zero and infinity (a transport fit may be zero, as for a species
+// that does not conduct); FP32 the correctly rounded ones.
+__device__ __forceinline__ double rule_rcp(double x) { return full_rcp(x); }
 __device__ __forceinline__ float rule_rcp(float x) { return 1 / x; }
-__device__ __forceinline__ double rule_sqrt(double x) { return x * fast_rsqrt(x); }
+__device__ __forceinline__ double rule_sqrt(double x) {
+    const double r = x * fast_rsqrt(x);
+    return r == r || x < 0 ? r : x;  // zero and infinity are their own roots
+}
 __device__ __forceinline__ float rule_sqrt(float x) { return sqrt(x); }
-__device__ __forceinline__ double rule_div(double a, double b) { return a * fast_rcp(b); }
+__device__ __forceinline__ double rule_div(double a, double b) { return a * full_rcp(b); }
 __device__ __forceinline__ float rule_div(float a, float b) { return a / b; }
 
 template <typename MT>
@@ -724,13 +728,13 @@ __device__ __forceinline__ void mixture_point(const FlameThermo &th, const Flame
                                               const MixTables<NS, MT> &mt, double T, double P,
                                               double rho_raw, const double *r, double &mu,
                                               double &lam, double *Dk) {
-    const double rhoinv = fast_rcp(jmax(rho_raw, kEps));
+    const double rhoinv = full_rcp(jmax(rho_raw, kEps));
     double X[NS];
     double yow = 0;
 #pragma unroll
     for (int n = 0; n < NS; ++n)
         X[n] = fast_div(jmax(r[n] * rhoinv, 0.0), th.mw[n]), yow += X[n];
-    const double yowinv = fast_rcp(yow);
+    const double yowinv = full_rcp(yow);
 #pragma unroll
     for (int n = 0; n < NS; ++n) X[n] *= yowinv;
     if constexpr (sizeof(MT) == 8) {

@@ -2,7 +2,8 @@
 
 The fused stages and the chemistry step divide by refined reciprocals.  A zero or infinite divisor
 has to give what the division gives: a species with a1 = 1 starts GetT from ein / 0 = inf
-(thermo.jl:231-282), Pr = inf switches conduction and diffusion off.  Bound: the fused FP64 stage's 1e-12
+(thermo.jl:231-282), Pr = inf switches conduction and diffusion off, and zero transport fits make
+single terms of mixtureProperties (thermo.jl:289-369) vanish.  Bound: the fused FP64 stage's 1e-12
 relative L2 per field, 1e-5 in mixed precision.
 """
 from __future__ import annotations
@@ -65,6 +66,26 @@ def test_infinite_prandtl_number(f3d, oracle, cuda_ok, ns, precision):
     dc = _agree(f3d, oracle, _case(f3d, ns, lambda th: tr), precision, 3, 1e-5 if precision else 1e-12)
     T = dc.T[dc.cur].cpu().numpy()
     assert (T[0] > 0).all() and (T[1] == 0).all() and (T[2] == 0).all()
+
+
+@pytest.mark.parametrize("ns", [1, 2, 9])  # every species everywhere: an absent one makes 0 / 0
+@pytest.mark.parametrize("zero", ["conductivity", "diffusion", "last viscosity"])
+def test_zero_transport_fits(f3d, oracle, cuda_ok, ns, zero):
+    if ns == 1 and zero == "diffusion":
+        pytest.skip("one species has no pair")
+
+    def transport(th):
+        tr = f3d.cases.mixture_averaged_transport(th, seed=5)
+        at = {"conductivity": slice(5 * ns, 10 * ns), "diffusion": slice(10 * ns, None),
+              "last viscosity": slice(5 * (ns - 1), 5 * ns)}[zero]
+        tr.poly[at] = 0.0
+        return tr
+
+    dc = _agree(f3d, oracle, _case(f3d, ns, transport), 0, 3, 1e-12)
+    T = dc.T[dc.cur].cpu().numpy()
+    assert np.isfinite(T).all()
+    if zero == "diffusion":
+        assert (T[2:] == 0).all()
 
 
 @pytest.mark.parametrize("stiff", [0, 1])
