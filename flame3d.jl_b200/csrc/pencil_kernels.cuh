@@ -73,6 +73,7 @@ struct Args {
     QT *aux;     // ϕ (1) and Y (NS), ghosted
     double *R;   // right-hand side accumulator (5 + NS), ghosted indexing: z sweep, then all
     double *R2;  // the y sweep's contribution (5 + NS), written, never read-modify-written
+    double *xq, *xs;  // FP64 sweeps: the x sweep's contribution, flow (5) and species (NS)
     FlameThermo th;
     FlameTransport tr;
 };
@@ -1064,6 +1065,7 @@ Args<QT> make_args(const FlameGrid &g, int stage, double dt, const FlameStageBuf
     A.R = static_cast<double *>(scratch);
     A.R2 = A.R + (size_t)(5 + g.ns) * A.np;
     A.aux = reinterpret_cast<QT *>(A.R2 + (size_t)(5 + g.ns) * A.np);
+    A.xq = sizeof(QT) == 8 ? static_cast<double *>(b.Q_out) : nullptr, A.xs = b.rhoi_out;
     A.th = th, A.tr = tr;
     return A;
 }
@@ -1125,28 +1127,65 @@ int launch_x(const Args<QT> &A, cudaStream_t s) {
     return flame_check_launch("flame_rk_stage (pencil)");
 }
 
+// Whether an output array is also one of those the finish reads (the last stage's result may go
+// where rhon was): then it cannot hold a sweep's part until the finish.
+template <typename QT>
+bool outputs_shared(const Args<QT> &A) {
+    const void *out[3] = {A.Qo, A.ro, A.To}, *kept[3] = {A.U, A.Un, A.rn};
+    for (const void *o : out)
+        for (const void *k : kept)
+            if (o == k) return true;
+    return false;
+}
+
+// R += R2, R2 = 0.
+static __global__ void __launch_bounds__(256) k_gather(double *R, double *R2, size_t n) {
+    for (size_t i = blockIdx.x * 256 + (size_t)threadIdx.x; i < n; i += 256 * (size_t)gridDim.x)
+        R[i] += R2[i], R2[i] = 0.0;
+}
+
 // FP64: prep, the three sweeps in one launch, finish; chained below 2^20 cells.
 inline bool chained(const Args<double> &A) { return (long long)A.nx * A.ny * A.nz < 1 << 20; }
 
+// The sweeps of an outputs_shared stage: z and y first, then x into R2, gathered into R in the same
+// order, so that the finish sums the same values (z + y) + x.
 template <int NS, bool MIXD>
-int launch_sweeps(const Args<double> &A, cudaStream_t s) {
+int launch_shared(const Args<double> &A, const SweepShape &P, cudaStream_t s) {
+    constexpr size_t sm = SweepSlots<NS, MIXD>::SMEM;
+    const size_t n = (size_t)(5 + NS) * A.np;
+    const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
+    SweepShape Px = P;
+    Px.y0 = Px.x0 = 0;
+    k_sweeps<NS, MIXD><<<(unsigned)P.x0, P.threads, sm, s>>>(A, P);
+    k_gather<<<blocks, 256, 0, s>>>(A.R, A.R2, n);
+    k_sweeps<NS, MIXD><<<(unsigned)(P.blocks - P.x0), P.threads, sm, s>>>(A, Px);
+    k_gather<<<blocks, 256, 0, s>>>(A.R, A.R2, n);
+    return flame_check_launch("flame_rk_stage (sweeps)");
+}
+
+template <int NS, bool MIXD>
+int launch_sweeps(const Args<double> &A, bool early, bool shared, cudaStream_t s) {
     constexpr size_t sm = SweepSlots<NS, MIXD>::SMEM;
     static std::atomic<bool> done[64];
     if (int e = set_smem(k_sweeps<NS, MIXD>, sm, done)) return e;
     const SweepShape P = sweep_shape<SweepSlots<NS, MIXD>>(A.nx, A.ny, A.nz);
-    return launch_chained(chained(A), k_sweeps<NS, MIXD>, P.blocks, P.threads, sm, s, "flame_rk_stage (sweeps)",
+    if (shared) return launch_shared<NS, MIXD>(A, P, s);
+    return launch_chained(early, k_sweeps<NS, MIXD>, P.blocks, P.threads, sm, s, "flame_rk_stage (sweeps)",
                           A, P);
 }
 template <int NS>
-int launch_fp64(const Args<double> &A, cudaStream_t s) {
+int launch_fp64(Args<double> A, cudaStream_t s) {
     k_prep<NS, double><<<(unsigned)((A.np + 255) / 256), 256, 0, s>>>(A);
     if (int e = flame_check_launch("flame_rk_stage (prep)")) return e;
     const unsigned blocks = (unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128);
+    const bool shared = outputs_shared(A), early = chained(A) && !shared;
+    if (shared) A.xq = A.R2, A.xs = A.R2 + 5 * (size_t)A.np;
     // law 2: per-species D_k (one species has the one D of the other laws)
-    if (int e = A.tr.law == 2 ? launch_sweeps<NS, (NS > 1)>(A, s) : launch_sweeps<NS, false>(A, s))
+    if (int e = A.tr.law == 2 ? launch_sweeps<NS, (NS > 1)>(A, early, shared, s)
+                              : launch_sweeps<NS, false>(A, early, shared, s))
         return e;
-    return launch_chained(chained(A),
-                          A.tr.law == 2 ? k_finish_mix<NS, double> : k_finish<NS, double, true>, blocks, 128, 0, s, "flame_rk_stage (finish)", A);
+    return launch_chained(early, A.tr.law == 2 ? k_finish_mix<NS, double> : k_finish<NS, double, true>,
+                          blocks, 128, 0, s, "flame_rk_stage (finish)", A);
 }
 
 // Mixed precision: the sweeps of sweep_kernels.cuh.
@@ -1187,6 +1226,7 @@ int launch_mixed(const Args<float> &A, cudaStream_t s, bool split_finish, bool s
         k_finish_mix<NS, T><<<blocks, 128, 0, s>>>(A);
         return flame_check_launch("flame_rk_stage (finish)");
     }
+    if (!MixedSlots<NS>::FIN && outputs_shared(A)) split_species = true;  // parts in R and R2 only
     if (split_species) {  // configurations 5, 6: flow sweep (the NS = 0 instance) + species sweep
         if (int e = launch_staged<2, 0, 0, T, T>(A, s)) return e;
         if (int e = launch_staged<2, 0, NS, T, T, 2>(A, s)) return e;

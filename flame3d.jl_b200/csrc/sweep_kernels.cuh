@@ -43,14 +43,14 @@ struct SweepSlots {
     static_assert(N <= MOST && MINB * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
 };
 
-// Where the x sweep leaves field n of a cell for the finish: the stage's output arrays, whose
-// interior the finish of the same cell writes after it has read this (rhoi_out one value of 8
-// bytes per species; for the five flow fields Q_out's seven).
+// Where the x sweep leaves field n of a cell for the finish (A.xq the five flow fields, A.xs the
+// species): the stage's output arrays, whose interior the finish of the same cell writes after it
+// has read this, or the second right-hand side (launch_shared).
 __device__ __forceinline__ void put_x(const Args<double> &A, int n, int c, double d) {
-    (n < 5 ? A.Qo + n * A.np : A.ro + (n - 5) * A.np)[c] = d;
+    (n < 5 ? A.xq + n * A.np : A.xs + (n - 5) * A.np)[c] = d;
 }
 __device__ __forceinline__ double get_x(const Args<double> &A, int n, int c) {
-    return (n < 5 ? A.Qo + n * A.np : A.ro + (n - 5) * A.np)[c];
+    return (n < 5 ? A.xq + n * A.np : A.xs + (n - 5) * A.np)[c];
 }
 
 // A block's lines and a thread's place in them: its point, its face (left of a cell) and the

@@ -375,7 +375,10 @@ int flame_rk_stage(const FlameGrid *g, flame_stream_t stream, int stage, double 
  * sweeps side by side, the finish (RK3 update, c2Prim, transport, ghosts); the interior of Q_out
  * and rhoi_out holds the x sweep's part between the last two.  In mixed precision 3 and 4 run
  * likewise (up to two species the x sweep is apart and finishes the stage; from three on the
- * interior of trans_out is used in between as well); one species on at least 2^20 cells takes
+ * interior of trans_out is used in between as well).  Where Q_out, rhoi_out or trans_out is one of
+ * U, Un and rhon (the last stage may leave its rhoi in rhon), nothing is left in them: FP64 runs
+ * the x sweep after the others, mixed precision from three species on configuration 5 or 6.
+ * Mixed precision with one species on at least 2^20 cells takes
  * four barrier-free launches (a prep pass and z, y, x warp-per-pencil sweeps, the x sweep
  * finishing the stage), with configuration 4 the finish in a fifth, bit-identical to 3;
  * 5, 6 = configurations 3, 4 with each z / y sweep split into a flow sweep and a species sweep
