@@ -1078,9 +1078,11 @@ int set_smem(K kernel, size_t sm, std::atomic<bool> *done) {
     // (two that both find the flag unset both set the attribute, to the same value)
     if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return FLAME_OK;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess) {
+        cudaGetLastError();
         return flame_fail(FLAME_ELAUNCH, "pencil sweep: %zu B shared memory: %s", sm,
                           cudaGetErrorString(e));
+    }
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return FLAME_OK;
 }
@@ -1096,9 +1098,7 @@ int launch_chained(bool early, void (*kernel)(P...), unsigned blocks, int thread
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     a.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &a, c.numAttrs = early ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, args...);
-    if (e != cudaSuccess)
-        return flame_fail(FLAME_ELAUNCH, "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
+    cudaLaunchKernelEx(&c, kernel, args...);  // an error is the thread's last, read and cleared here
     return flame_check_launch(what);
 }
 
@@ -1340,8 +1340,10 @@ int batch_launch(const BatchChunk &bc, cudaStream_t s, int stage, int parity, in
                                              cudaMemcpyDeviceToDevice, s);
     if (ce == cudaSuccess)
         ce = cudaMemsetAsync(bc.counters, 0, sizeof(int) * (4 + 4 * (size_t)bc.n), s);
-    if (ce != cudaSuccess)
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
         return flame_fail(FLAME_ELAUNCH, "flame_batch_stage: %s", cudaGetErrorString(ce));
+    }
     BatchLaunch L;
     L.items = bc.items;
     L.need = bc.need;

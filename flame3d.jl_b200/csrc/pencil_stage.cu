@@ -152,6 +152,14 @@ struct Layout {
     size_t bytes = 0;
 };
 
+// The status of a runtime call.  A failed call also leaves its error as the thread's last one, which
+// the next launch check would report as its own, so it is cleared.
+int batch_error(cudaError_t e, const char *what) {
+    if (e == cudaSuccess) return FLAME_OK;
+    cudaGetLastError();
+    return flame_fail(FLAME_ELAUNCH, "%s: %s", what, cudaGetErrorString(e));
+}
+
 // Lanes of a batch.  Small cases leave the GPU idle between and inside their chunks' launches:
 // ten cases of 32^3 and 48^3 with four species counts 1868 -> 1772 us a step, six of 33^3 to 60^3 1872
 // -> 1652, six of 48^3 to 96^3 (2.7 million cells) 4190 -> 4122.  Beyond 2^22 cells a batch fills the
@@ -175,9 +183,7 @@ int make_lanes(FlameBatch &B, long long cells) {
         e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e == cudaSuccess) B.joined.push_back(ev);
     }
-    if (e != cudaSuccess)
-        return flame_fail(FLAME_ELAUNCH, "flame_batch_create: %s", cudaGetErrorString(e));
-    return FLAME_OK;
+    return batch_error(e, "flame_batch_create");
 }
 
 // A case's group: its species count, and whether it has per-species D_k (law 2).
@@ -333,9 +339,9 @@ extern "C" int flame_batch_create(FlameBatch **out, const FlameCaseDesc *cases, 
     }
     cudaError_t ce = cudaMemcpyAsync(workspace, host.data(), L.bytes, cudaMemcpyHostToDevice, s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-    if (ce != cudaSuccess) {
+    if (int e = batch_error(ce, "flame_batch_create: upload")) {
         delete B;
-        return flame_fail(FLAME_ELAUNCH, "flame_batch_create: upload: %s", cudaGetErrorString(ce));
+        return e;
     }
     *out = B;
     return FLAME_OK;
@@ -361,10 +367,8 @@ extern "C" int flame_batch_stage(FlameBatch *B, flame_stream_t s, int stage, int
         if (je == cudaSuccess) je = cudaStreamWaitEvent(s, B->joined[k], 0);
         if (ce == cudaSuccess) ce = je;
     }
-    if (err) return err;
-    if (ce != cudaSuccess)
-        return flame_fail(FLAME_ELAUNCH, "flame_batch_stage: %s", cudaGetErrorString(ce));
-    return FLAME_OK;
+    if (ce != cudaSuccess) cudaGetLastError();
+    return err ? err : batch_error(ce, "flame_batch_stage");
 }
 
 extern "C" int flame_batch_status(FlameBatch *B, flame_stream_t s) {
@@ -374,8 +378,7 @@ extern "C" int flame_batch_status(FlameBatch *B, flame_stream_t s) {
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
     if (ce == cudaSuccess && h) ce = cudaMemsetAsync(B->err, 0, sizeof(int), s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-    if (ce != cudaSuccess)
-        return flame_fail(FLAME_ELAUNCH, "flame_batch_status: %s", cudaGetErrorString(ce));
+    if (int e = batch_error(ce, "flame_batch_status")) return e;
     if (h)
         return flame_fail(FLAME_ETIMEOUT,
                           "flame_batch_stage: a wait for another work item's completion ran out; "
