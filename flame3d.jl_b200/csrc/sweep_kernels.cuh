@@ -356,16 +356,22 @@ struct MixedSlots {
 };
 
 // The x sweep's FP64 flow differences as pairs of 32-bit words in Q_out's seven fields and the
-// transport's three.
-__device__ __forceinline__ int *x_word(const Args<float> &A, int k, int c) {
-    return reinterpret_cast<int *>(k < 7 ? A.Qo + k * A.np + c : A.To + (k - 7) * A.np + c);
+// transport's three (as floats of the same bits, so that the compiler sees the type that the finish
+// stores there).
+__device__ __forceinline__ float *x_word(const Args<float> &A, int k, int c) {
+    return k < 7 ? A.Qo + k * A.np + c : A.To + (k - 7) * A.np + c;
 }
 __device__ __forceinline__ void put_x(const Args<float> &A, int n, int c, double d) {
-    if (n < 5) *x_word(A, 2 * n, c) = __double2loint(d), *x_word(A, 2 * n + 1, c) = __double2hiint(d);
-    else A.ro[(n - 5) * A.np + c] = d;
+    if (n < 5) {
+        *x_word(A, 2 * n, c) = __int_as_float(__double2loint(d));
+        *x_word(A, 2 * n + 1, c) = __int_as_float(__double2hiint(d));
+    } else {
+        A.ro[(n - 5) * A.np + c] = d;
+    }
 }
 __device__ __forceinline__ double get_x(const Args<float> &A, int n, int c) {
-    return n < 5 ? __hiloint2double(*x_word(A, 2 * n + 1, c), *x_word(A, 2 * n, c))
+    return n < 5 ? __hiloint2double(__float_as_int(*x_word(A, 2 * n + 1, c)),
+                                    __float_as_int(*x_word(A, 2 * n, c)))
                  : A.ro[(n - 5) * A.np + c];
 }
 
@@ -596,4 +602,4 @@ __global__ void __launch_bounds__(MixedSlots<NS>::NT, MixedSlots<NS>::MINB)
 }
 
 // Mixed precision: one species on at least 2^20 cells runs the staged sweeps (figures above).
-inline bool staged_sweeps_ahead(int ns, long long cells) { return ns == 1 && cells >= 1 << 20; }
+constexpr bool staged_sweeps_ahead(int ns, long long cells) { return ns == 1 && cells >= 1 << 20; }
