@@ -133,6 +133,7 @@ SIGNATURES = {
     "flame_rk_stage_noalloc": [G, S, I, D, C.POINTER(FlameStageBuffers), M, TH, TR, I],
     "flame_transport": [G, S, P, P, P, TH, TR, I],
     "flame_transport_boundary": [G, S, P, P, P, TH, TR, I],
+    "flame_stage_launches": [I, C.c_longlong, I, I, I],
     "flame_stage_scratch_bytes": [G, I],
     "flame_batch_workspace_bytes": [C.POINTER(FlameCaseDesc), I, I],
     "flame_batch_create": [C.POINTER(C.c_void_p), C.POINTER(FlameCaseDesc), I, I, P, C.c_size_t,

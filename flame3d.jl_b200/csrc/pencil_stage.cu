@@ -42,6 +42,21 @@ int flame_pencil_stage(const FlameGrid *g, cudaStream_t s, int stage, double dt,
                                  split_species != 0);
 }
 
+// What launch_fp64 and launch_mixed issue.
+extern "C" int flame_stage_launches(int ns, long long cells, int law, int precision, int tile) {
+    const bool tiled = tile >= 0 && tile <= 2;
+    if (ns < 1 || ns > FLAME_FUSED_MAX_NS || cells < 1 || law < 0 || law > 2 || tile < 0 || tile > 6 ||
+        (precision != 0 && precision != 1) || (tiled && law == 2))
+        return 0;
+    if (tiled) return 1;
+    if (precision == 0) return 3;                // prep, the sweeps, finish
+    if (law == 2) return 7;                      // prep, flow and species sweeps of z and y, x, finish
+    const int finish = tile == 4 || tile == 6;
+    if (tile >= 5) return 6 + finish;
+    if (!flame::pencil::staged_sweeps_ahead(ns, cells)) return 3;
+    return 4 + finish;                           // prep, z, y, x
+}
+
 // SIZE_MAX when the product does not fit in size_t (then no buffer can be large enough).
 extern "C" size_t flame_stage_scratch_bytes(const FlameGrid *g, int precision) {
     if (!g || g->nx < 1 || g->ny < 1 || g->nz < 1 || g->ng < 0 || g->ns < 0) return 0;

@@ -258,28 +258,31 @@ class DeviceCase:
             return 6
         return self.tile
 
+    def launches_per_stage(self, tile: int | None = None) -> int:
+        """Kernels one fused stage launches (of configuration `tile` instead of the case's own): 1
+        for a tile kernel, 3 for the sweeps in one launch, 4 to 7 for the staged sweeps."""
+        return self.lib.flame_stage_launches(self.case.ns, self.case.cells, self.transport.law,
+                                             self.precision, self.tile if tile is None else tile)
+
     @property
     def swept(self) -> bool:
-        """Whether a pencil configuration runs the sweeps of sweep_kernels.cuh: all of FP64; in
-        mixed precision configurations 3 and 4 but for one species on at least 2^20 cells."""
-        t = self.launched_config
-        if self.precision == 0:
-            return t in (3, 4, 5, 6)
-        return t in (3, 4) and (self.case.ns > 1 or self.case.cells < 1 << 20)
+        """Whether a pencil configuration runs the sweeps of sweep_kernels.cuh (three launches)."""
+        return self.tile in (3, 4, 5, 6) and self.launches_per_stage() == 3
 
-    def launches_per_stage(self) -> int:
-        """Kernels one fused stage launches: 1 for a tile kernel, 3 for the sweeps in one launch;
-        with the staged sweeps 4, one more with the separate finish (4, 6) and two more with
-        split species sweeps (5, 6)."""
-        if self.swept:
-            return 3
-        return {3: 4, 4: 5, 5: 6, 6: 7}.get(self.launched_config, 1)
+    def same_launches(self, tile: int) -> int:
+        """The lowest configuration with the launches of `tile`: of the pencil configurations, one
+        with as many kernels."""
+        if tile not in (3, 4, 5, 6):
+            return tile
+        n = self.launches_per_stage(tile)
+        return next(t for t in (3, 4, 5, 6) if self.launches_per_stage(t) == n)
 
     def stage_kernels(self) -> str:
         t = self.launched_config
         if self.swept:
             if self.precision == 0:
-                return "pencil::k_prep + k_sweeps<z, y, x> + k_finish"
+                return ("pencil::k_prep + k_sweeps<z, y, x> + "
+                        + ("k_finish_mix" if self.transport.law == 2 else "k_finish"))
             return ("pencil::k_prep + k_sweeps_mixed<z, y> + k_sweep_x_finish" if self.case.ns <= 2
                     else "pencil::k_prep + k_sweeps_mixed<z, y, x> + k_finish")
         if t in (3, 4, 5, 6):

@@ -394,6 +394,11 @@ int flame_rk_stage_tiled(const FlameGrid *g, flame_stream_t stream, int stage, d
                          const FlameThermo *thermo, const FlameTransport *transport,
                          int precision, int tile);
 
+/* Kernels that one stage of a configuration launches (0: the stage refuses it), for grids of `cells`
+ * interior cells and transport law `law`, with output buffers that are none of U, Un and rhon.  Of
+ * configurations 3 to 6 those with equal counts launch the same kernels. */
+int flame_stage_launches(int ns, long long cells, int law, int precision, int tile);
+
 /* Bytes of scratch the pencil configurations need: 2 (5 + ns) doubles (the right-hand side of
  * the z sweep and of the y sweep) and (1 + ns) values of the storage type per ghosted point. */
 size_t flame_stage_scratch_bytes(const FlameGrid *g, int precision);
