@@ -1,18 +1,21 @@
 """Autotuner: picks the stage configuration per (GPU, precision, species count, grid size).
 
 Configurations (flame_rk_stage_tiled): 0, 1, 2 = one tile kernel per stage (16x8x8 with one or
-two CTAs per SM, 8x8x8); 3 = prep + z, y, x pencil sweeps, the x sweep finishing the stage;
-4 = the same sweeps with the finish in its own per-cell launch; 5, 6 = 3, 4 with each y / z
-sweep split into a flow sweep and a species sweep.  The mixture-averaged transport (law 2) runs
-on the pencil configurations only (as 6); the tile configurations refuse it and are skipped.  Which is fastest depends on
-the species count (registers and shared memory per point grow with it), on the grid size (the
-tile kernels launch once per stage, which matters for small grids) and on the precision.
+two CTAs per SM, 8x8x8); 3 to 6 = the sweeps along the grid axes, in FP64 all the same launches, in
+mixed precision the sweeps in one launch (3, 4) or apart (5, 6, the species in sweeps of their own;
+4, 6 and, for one species on large grids, 4 with a separate finish).  The mixture-averaged transport
+(law 2) runs on 3 to 6 only, always with the same launches; the tile configurations refuse it and are
+skipped.  Which is fastest depends on the species count (registers and shared memory per point grow
+with it), on the grid size (the tile kernels launch once per stage, which matters for small grids)
+and on the precision.
 
 The tuner times every candidate on a device-side clone of the case being set up (its own
 fields, so the hybrid scheme's branch mix is the real one), a warm-up step and then `steps`
-timed RK3 steps with CUDA events, and keeps the fastest.  Choices are cached in a JSON file
-(FLAME3D_B200_CACHE, else ~/.cache/flame3d_b200/autotune.json) under a key naming the GPU,
-precision, species count and the grid's size class (log2 of the cell count).
+timed RK3 steps with CUDA events, and keeps the fastest; of configurations that launch the same
+kernels only the lowest is timed.  Choices are cached in a JSON file (FLAME3D_B200_CACHE, else
+~/.cache/flame3d_b200/autotune.json) under a key naming the GPU, the generation of the kernels, the
+precision, species count and the grid's size class (log2 of the cell count, split where the
+library changes kernels inside a class).
 """
 from __future__ import annotations
 
@@ -22,7 +25,10 @@ import os
 import threading
 from pathlib import Path
 
+from . import abi
+
 CANDIDATES = (0, 1, 2, 3, 4, 5, 6)
+GENERATION = 2  # raised when the kernels of a configuration change: older choices are timed again
 
 
 def cache_path() -> Path:
@@ -37,8 +43,11 @@ def size_class(cells: int) -> int:
 
 def key(gpu: str, precision: int, ns: int, cells: int, law: int = 1) -> str:
     """The cache key; the mixture-averaged transport (law 2) is tuned apart (its candidates and
-    its costs differ)."""
-    return f"{gpu}|p{precision}|ns{ns}|c{size_class(cells)}" + ("|law2" if law == 2 else "")
+    its costs differ), and so are the two sides of a size at which configuration 3 changes kernels
+    (mixed precision, one species)."""
+    kernels = abi.load_library().flame_stage_launches(ns, cells, law, precision, 3)
+    return (f"{gpu}|g{GENERATION}|p{precision}|ns{ns}|c{size_class(cells)}|k{kernels}"
+            + ("|law2" if law == 2 else ""))
 
 
 class Autotuner:
@@ -87,7 +96,8 @@ class Autotuner:
             if hit is not None:
                 return int(hit["tile"])
             times = {}
-            for t in self.candidates:
+            same = getattr(dc, "same_launches", lambda t: t)
+            for t in dict.fromkeys(same(t) for t in self.candidates):
                 try:
                     times[t] = float(self.measure(dc, t))
                 except Exception:  # a configuration that cannot run this case is skipped
