@@ -110,7 +110,8 @@ class Batch:
         Flips the graph part's cases (as DeviceCase.step does), not the persistent part's."""
         main = torch.cuda.current_stream(self.device)
         parts = list(self.parts)
-        if parts and parts[0].mode == "persistent":
+        beside = parts[0].mode == "persistent"
+        if beside:
             pers = parts.pop(0)
             ev = torch.cuda.Event()
             ev.record(main)
@@ -122,7 +123,8 @@ class Batch:
                     p ^= 1
         for part in parts:  # the graph part forks from and joins back to `main` itself
             part._fork_step()
-        main.wait_stream(self.pstream)
+        if beside:  # a stream that the capture never forked cannot be joined to it
+            main.wait_stream(self.pstream)
 
     def _hybrid_flip(self) -> None:
         """The bookkeeping of one step: the persistent part's three stage flips (its graph
