@@ -79,9 +79,10 @@ __device__ __forceinline__ double fast_div(double a, double b) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
     const double e = fma(-b, x, 1.0), r = fma(x, fma(e, e, e), x), q = a * r;
     const double c = fma(fma(-b, q, a), r, q);
-    return c == c ? c : a * x;
+    return c == c && q != 0 ? c : a * x;  // a zero's sign is the seed's too
 }
-// x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2
+// x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2, the series of x / sqrt(1 - e) cut after the second
+// order.  The rounding of d x leaves 2^-54 before that of the last multiply-add.
 __device__ __forceinline__ double fast_rsqrt(double d) {
     double x;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
@@ -339,8 +340,8 @@ __device__ __forceinline__ T nmax(T a, T b) {
 // from 6.75 to 6.34 ms, 101x75x63 with five species from 2.00 to 1.80 ms, 32^3 from 139 to 129 us.
 //
 // Σ α_k r_k / Σ α_k comes as a fraction N / D without divisions: multiplying every α_k by
-// b_1^2 b_2^2 b_3^2 gives A_k = d_k (b_k^2 + τ^2) Π_{j≠k} b_j^2 with the same ratios (the
-// products stay in range for |β| < 1e49).
+// b_1^2 b_2^2 b_3^2 gives A_k = d_k (b_k^2 + τ^2) Π_{j≠k} b_j^2 with the same ratios (N, of
+// the order of 144 (4β)^6 sqrt(β), stays in range for β < 1e46).
 __device__ __forceinline__ void weno_fraction(double V1, double V2, double V3, double V4,
                                               double V5, double &N, double &D) {
     const double e1 = V2 - V1, e2 = V3 - V2, e3 = V4 - V3, e4 = V5 - V4;
