@@ -807,7 +807,7 @@ def main() -> int:
                         "peak_source": "measured (csrc/probe/fp64_peak.cu, this run)",
                         "counts_source": counts.get("source")}
         roof["limiter"] = ("neither roof: latency and barriers at 24 of 64 warps per SM in the "
-                           "sweeps (profiles/sweeps_jet128x64x64_fp64.md)")
+                           "sweeps")
 
     cpu = None
     if not args.no_cpu:

@@ -6,10 +6,12 @@
 // Rates follow vproductionRate / vproductionRate_Jac: Arrhenius forward rates, equilibrium
 // constants from the Gibbs energy (thermo.jl:163-191), third-body and Troe falloff reactions.
 //
-// Built with -fmad=false, like kernels_ref.cu: apart from exp / log / pow (the device math
-// library against the host's) the arithmetic is the oracle's, operation by operation.  One
-// thread per cell; the per-cell work arrays (ns, nreacs and ns x ns doubles) live in local
-// memory, as MVector / MMatrix do in the reference.
+// Built with -fmad=false, like kernels_ref.cu.  One thread per cell.  Above nine species the
+// arithmetic is the oracle's, operation by operation, apart from exp / log / pow (the device math
+// library against the host's), and the work arrays (ns, nreacs and ns x ns doubles) live in local
+// memory, as MVector / MMatrix do in the reference.  Up to nine they live in registers, and
+// reciprocals stand for some divisions, the elimination is written with fma and T comes from the
+// mixture's polynomial: within 1e-12 of the oracle (tests/test_parity_chemistry.py).
 
 #include "common.cuh"
 

@@ -1,4 +1,4 @@
-// sweep_kernels.cuh — the three FP64 sweeps of a stage in one launch (sm_100a).
+// sweep_kernels.cuh — the three sweeps of a stage in one launch, FP64 and mixed precision (sm_100a).
 //
 // A block takes a few lines of points along its sweep axis: eight neighbouring x columns of up to
 // 32 points (y and z sweeps), or a few whole or cut rows (x sweep).  A thread owns one point of
@@ -18,7 +18,8 @@
 // Bound by latency at 24 warps per SM (128x64x64 jet: 0.40 instructions per scheduler and cycle,
 // FP64 pipe 41 %; barrier and long-scoreboard stalls lead), with 2000 instruction slots per cell
 // and sweep where a warp per 32-point pencil took 3137.  One step, before -> after: 32^3 135 ->
-// 92 us, 64^3 521 -> 402, 128^3 2896 -> 2584, jet 256x128x128 6380 -> 6313; 101x75x63 with five
+// 92 us, 64^3 521 -> 402, 128^3 2896 -> 2584, jet 256x128x128 6380 -> 5780 (its x blocks then hold
+// five rows of 49 points; with one row of 92 in 256 threads 6313); 101x75x63 with five
 // species 1784 -> 1061; 96^3 with nine species 5415 -> 2741, with per-species D 4638 -> 4019.
 // Tried and not kept: two blocks per SM at 128 registers (jet 6623) and four at 64 (7810);
 // everything but the metrics staged in pass 1 (6920); a prefetch of pass 2's lines to L2 (6399).
