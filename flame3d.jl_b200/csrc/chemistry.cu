@@ -231,6 +231,7 @@ __device__ __forceinline__ void fill_tables(MechTables<NS> &t, const Mech &M,
                                             const FlameThermo &th) {
     for (int n = threadIdx.x; n < M.nr; n += blockDim.x) {
         unsigned fm = 0, rm = 0;
+        const int type = (int)M.type[n];
         for (int m = 0; m < NS; ++m) {
             const long long vf = M.vf[m + NS * n], vr = M.vr[m + NS * n];
             t.vf[n][m] = vf, t.vr[n][m] = vr;
@@ -238,7 +239,6 @@ __device__ __forceinline__ void fill_tables(MechTables<NS> &t, const Mech &M,
             fm |= (vf != 0 ? 1u : 0u) << m, rm |= (vr != 0 ? 1u : 0u) << m;
         }
         t.fmask[n] = fm, t.rmask[n] = rm;
-        const int type = (int)M.type[n];
         t.type[n] = type, t.sgm[n] = M.sgm[n];
         for (int a = 0; a < 3; ++a) t.Arr[n][a] = M.Arr[3 * n + a];
         // only what the reaction's type uses is read, so the arrays may end with the last reaction
@@ -380,8 +380,9 @@ __global__ void __launch_bounds__(128) k_eval_ns(Dims D, double *U, double *Q, d
     if (hot) T = Q[p + 5 * np], hot = T > Tcrit;
     // A block without a hot cell leaves the mechanism alone.  Eight species, 96^3 cells, explicit /
     // point-implicit: no cell hot 25 / 33 -> 13 / 19 us (the run-time kernel, with fewer registers,
-    // 15 / 15), one cell in a hundred 110 / 205 -> 87 / 181, all of them 310 / 640 -> 296 / 635.  A
-    // loop over chunks in as many blocks as the GPU holds spills (all hot 352 / 691).
+    // 15 / 15), one cell in a hundred 110 / 205 -> 87 / 179, all of them 310 / 640 -> 296 / 635; a grid
+    // of a few blocks pays the load of T first (16^3 27.1 -> 28.0).  A loop over chunks in as many
+    // blocks as the GPU holds spills (all hot 352 / 691).
     if (!__syncthreads_or(hot)) return;
     fill_tables<NS>(t, M, th);
     __syncthreads();

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/flame3d_b200.h"
 
@@ -71,15 +72,19 @@ __device__ __forceinline__ double full_rcp(double d) {
 // a / b: the quotient by the refined reciprocal and one correction from its residual (P. Markstein,
 // Computation of elementary functions on the IBM RISC System/6000 processor, 1990), which leaves it
 // within rounding of the correctly rounded one (no branch and no call, so a kernel near its register
-// limit does not spill around it).  A zero or infinite operand, or a quotient that overflows, gives
-// what a division gives, by the seed; a quotient or reciprocal below the normal range may come out
-// as zero.
+// limit does not spill around it).  b is normal with a normal reciprocal, a finite.
 __device__ __forceinline__ double fast_div(double a, double b) {
+    const double r = fast_rcp(b), q = a * r;
+    return fma(fma(-b, q, a), r, q);
+}
+// The same for any operands: a zero or infinite one, or a quotient that overflows, gives what a
+// division gives, by the seed; a quotient or reciprocal below the normal range may come out as zero.
+__device__ __forceinline__ double full_div(double a, double b) {
     double x;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
     const double e = fma(-b, x, 1.0), r = fma(x, fma(e, e, e), x), q = a * r;
     const double c = fma(fma(-b, q, a), r, q);
-    return c == c && q != 0 ? c : a * x;  // a zero's sign is the seed's too
+    return fabs(c) > 0 ? c : a * x;  // not a number, or a zero, whose sign is the seed's too
 }
 // x (1 + e/2 + 3 e^2 / 8) with e = 1 - d x^2, the series of x / sqrt(1 - e) cut after the second
 // order.  The rounding of d x leaves 2^-54 before that of the last multiply-add.
@@ -238,8 +243,9 @@ __device__ double get_T_mix(const MixPoly<NS> &M, const FlameThermo &th, double 
     const double emin = M.e(tmin), emax = M.e(tmax);
     if (ein < emin) return tmin - (emin - ein) / M.cv(tmin);
     if (ein > emax) return tmax - (emax - ein) / M.cv(tmax);
-    double t1 = ein * full_rcp(M.lo[0] * th.Ru);  // Σ_n (a1_n - 1) Ru / W_n ρ_n is the mixture's own
-    if (t1 < tmin || t1 > tmax) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
+    // Σ_n (a1_n - 1) Ru / W_n ρ_n is the mixture's own; where it is zero ein / 0 lies outside as well
+    double t1 = ein * fast_rcp(M.lo[0] * th.Ru);
+    if (!(t1 >= tmin && t1 <= tmax)) t1 = tmin + (tmax - tmin) / (emax - emin) * (ein - emin);
     for (int it = 0; it < 30; ++it) {
         double dt = (ein - M.e(t1)) * full_rcp(M.cv(t1));
         if (dt > 100.0)
@@ -646,22 +652,64 @@ __device__ __forceinline__ void mix_tables_fill(const FlameThermo &th, const Fla
     }
 }
 
-// Reciprocal, square root and quotient of the mixture rule: FP64 by the refined forms, with what
-// the exact operations give for zero and infinity (a transport fit may be zero, as for a species
-// that does not conduct); FP32 the correctly rounded ones.
-__device__ __forceinline__ double rule_rcp(double x) { return full_rcp(x); }
+// Reciprocal, square root and quotient of the mixture rule: FP64 by the refined forms (arguments
+// are positive and normal; mixture_exact has the other cases), FP32 the correctly rounded ones.
+__device__ __forceinline__ double rule_rcp(double x) { return fast_rcp(x); }
 __device__ __forceinline__ float rule_rcp(float x) { return 1 / x; }
-__device__ __forceinline__ double rule_sqrt(double x) {
-    const double r = x * fast_rsqrt(x);
-    return r == r || x < 0 ? r : x;  // zero and infinity are their own roots
-}
+__device__ __forceinline__ double rule_sqrt(double x) { return x * fast_rsqrt(x); }
 __device__ __forceinline__ float rule_sqrt(float x) { return sqrt(x); }
-__device__ __forceinline__ double rule_div(double a, double b) { return a * full_rcp(b); }
+__device__ __forceinline__ double rule_div(double a, double b) { return a * fast_rcp(b); }
 __device__ __forceinline__ float rule_div(float a, float b) { return a / b; }
 
 template <typename MT>
 __device__ __forceinline__ MT dot5t(MT l1, MT l2, MT l3, MT l4, const MT *p) {
     return p[0] + l1 * p[1] + l2 * p[2] + l3 * p[3] + l4 * p[4];
+}
+
+// mixture_properties_pairs with exact divisions and square roots, for a point where its refined ones
+// gave a value that is not a number: a transport fit may be zero (a species that does not conduct or
+// diffuse), and exact divisions then make terms zero or infinite and the result finite.  A function of
+// its own, since guarding each operation costs a step of 64x40x36 cells with nine species 4 % and the
+// same code a second time in the caller makes it spill.  out: λ, μ, D_0 .. D_{NS-1}.
+template <int NS>
+__device__ __noinline__ void mixture_exact(double T, double P, const double *X, const double *pw,
+                                           const double *poly, double *out) {
+    const double *visc = poly, *cond = poly + 5 * NS, *bin = poly + 10 * NS;
+    const double sqT = sqrt(T), sqsqT = sqrt(sqT), lgT = log(T);
+    const double lgT2 = lgT * lgT, lgT3 = lgT * lgT2, lgT4 = lgT2 * lgT2;
+    double mui[NS];
+    double sum1 = 0, sum2 = 0;
+    for (int k = 0; k < NS; ++k) {
+        const double c = sqT * dot5(lgT, lgT2, lgT3, lgT4, cond + 5 * k);
+        sum1 += X[k] * c, sum2 += X[k] / c;
+    }
+    out[0] = 0.5 * (sum1 + 1 / sum2);
+    for (int n = 0; n < NS; ++n) {
+        const double s = sqsqT * dot5(lgT, lgT2, lgT3, lgT4, visc + 5 * n);
+        mui[n] = s * s;
+    }
+    double mu = 0;
+    for (int n = 0; n < NS; ++n) {
+        double row = 0;
+        for (int l = 0; l < NS; ++l) {
+            // the pair's factor t = W[hi][lo] with hi > lo, and W[lo][hi] = t / (vr wr)
+            const int hi = n > l ? n : l, lo = n > l ? l : n, i = hi * NS + lo;
+            const double vr = mui[hi] / mui[lo], f1 = 1 + sqrt(vr * pw[NS * NS + i]);
+            const double t = f1 * f1 * pw[2 * NS * NS + i];
+            row += X[l] * (l == n ? 1.0 : l < n ? t : t / vr * pw[i]);
+        }
+        mu += X[n] * mui[n] / row;
+    }
+    out[1] = mu;
+    for (int n = 0; n < NS; ++n) {
+        double row = 0;
+        for (int m = 0; m < NS; ++m) {
+            if (m == n) continue;
+            const int hi = n > m ? n : m, lo = n > m ? m : n;
+            row += X[m] / (T * sqT * dot5(lgT, lgT2, lgT3, lgT4, bin + 5 * (hi + NS * lo)));
+        }
+        out[2 + n] = (1 - X[n]) / (row * P + kEps);
+    }
 }
 
 template <int NS, typename MT>
@@ -719,6 +767,20 @@ __device__ __forceinline__ void mixture_properties_pairs(MT T, MT P, const MT *X
         const MT s = row[n] * P;
         Dk[n] = rule_div(1 - X[n], s + MT(kEps));
     }
+    if constexpr (sizeof(MT) == 8) {
+        MT all = lam + mu;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) all += Dk[n];
+        if (__builtin_expect(all != all, 0)) {
+            double x[NS], out[2 + NS];
+#pragma unroll
+            for (int n = 0; n < NS; ++n) x[n] = X[n];
+            mixture_exact<NS>(T, P, x, pw, poly, out);
+            lam = out[0], mu = out[1];
+#pragma unroll
+            for (int n = 0; n < NS; ++n) Dk[n] = out[2 + n];
+        }
+    }
 }
 
 // The reference's mixture kernel at one point with law 2 (thermo.jl:371-403): Y = max(ρi/ρ, 0)
@@ -729,13 +791,13 @@ __device__ __forceinline__ void mixture_point(const FlameThermo &th, const Flame
                                               const MixTables<NS, MT> &mt, double T, double P,
                                               double rho_raw, const double *r, double &mu,
                                               double &lam, double *Dk) {
-    const double rhoinv = full_rcp(jmax(rho_raw, kEps));
+    const double rhoinv = fast_rcp(jmax(rho_raw, kEps));
     double X[NS];
     double yow = 0;
 #pragma unroll
     for (int n = 0; n < NS; ++n)
         X[n] = fast_div(jmax(r[n] * rhoinv, 0.0), th.mw[n]), yow += X[n];
-    const double yowinv = full_rcp(yow);
+    const double yowinv = fast_rcp(yow);
 #pragma unroll
     for (int n = 0; n < NS; ++n) X[n] *= yowinv;
     if constexpr (sizeof(MT) == 8) {

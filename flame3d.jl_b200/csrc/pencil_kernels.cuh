@@ -537,9 +537,9 @@ __device__ __forceinline__ void finish_cell(const Args<QT> &A, int g, int gx, in
                 mu = A.tr.mu_ref, lam = A.tr.lambda_ref, D = A.tr.D_ref;
             } else {  // transport_point with cp_mix = Σ_n w_n cp_n / ρ from the same polynomials
                 const double rcp = M.cv(Tn) + A.th.Ru * M.wsum;  // ρ cp
-                mu = A.tr.mu_ref * pow(fast_div(Tn, A.tr.T_ref), A.tr.exponent);
-                lam = fast_div(rcp * rinv * mu, A.tr.Pr);
-                D = fast_div(lam, rcp);
+                mu = A.tr.mu_ref * pow(full_div(Tn, A.tr.T_ref), A.tr.exponent);
+                lam = full_div(rcp * rinv * mu, A.tr.Pr);
+                D = full_div(lam, rcp);
             }
         }
     }
@@ -1174,12 +1174,16 @@ int launch_sweeps(const Args<double> &A, bool early, bool shared, cudaStream_t s
                           A, P);
 }
 template <int NS>
-int launch_fp64(Args<double> A, cudaStream_t s) {
+int launch_fp64(const Args<double> &A, cudaStream_t s, bool shared = false) {
+    if (!shared && outputs_shared(A)) {
+        Args<double> B = A;
+        B.xq = A.R2, B.xs = A.R2 + 5 * (size_t)A.np;
+        return launch_fp64<NS>(B, s, true);
+    }
     k_prep<NS, double><<<(unsigned)((A.np + 255) / 256), 256, 0, s>>>(A);
     if (int e = flame_check_launch("flame_rk_stage (prep)")) return e;
     const unsigned blocks = (unsigned)(((long long)A.nx * A.ny * A.nz + 127) / 128);
-    const bool shared = outputs_shared(A), early = chained(A) && !shared;
-    if (shared) A.xq = A.R2, A.xs = A.R2 + 5 * (size_t)A.np;
+    const bool early = chained(A) && !shared;
     // law 2: per-species D_k (one species has the one D of the other laws)
     if (int e = A.tr.law == 2 ? launch_sweeps<NS, (NS > 1)>(A, early, shared, s)
                               : launch_sweeps<NS, false>(A, early, shared, s))

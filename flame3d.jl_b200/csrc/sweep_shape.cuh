@@ -1,6 +1,8 @@
 // sweep_shape.cuh — how a launch of the sweeps (sweep_kernels.cuh) is cut into blocks.  Host code.
 #pragma once
 
+#include <algorithm>
+
 namespace flame {
 namespace pencil {
 
@@ -33,31 +35,34 @@ inline SweepShape sweep_shape(int nx, int ny, int nz) {
         const int nseg = (ext[d] + most - 1) / most;
         P.own[d] = (ext[d] + nseg - 1) / nseg;
     }
-    const long long all = ny * (long long)nz;
+    const int all = ny * nz;  // rows; the grid's points fit in 31 bits
     constexpr int kPlaces = 148 * SL::MINB;
-    struct Cut {
-        int own = 0, rows = 0;
-        long long warps = 0, blocks = 0;
-    } full, least;  // warps and blocks of `full` per `rows` rows, of `least` per launch
+    int own_full = 0, rows_full = 0, warps_full = 0, blocks_full = 0;  // per rows_full rows
+    int own_least = 0, rows_least = 0;
+    long long least = 0;                          // warps of the whole launch
     const int fewest = (nx + NT - 7) / (NT - 6);  // cuts with which a row fits a block
-    for (int nseg = fewest; nseg <= fewest + 24 && nseg <= (nx + 25) / 26 + 1; ++nseg) {
-        const int own = (nx + nseg - 1) / nseg;
-        for (int rows = 1; rows * (own + 6) <= NT; ++rows) {
-            const long long s = (nx + own - 1) / own;
-            const long long w = s * ((rows * (own + 6) + 31) / 32 + (rows * (own + 1) + 31) / 32);
-            const long long more = w * full.rows - full.warps * rows;  // > 0: more warps per row
-            if (!full.rows || more < 0 || (more == 0 && s * full.rows < full.blocks * rows))
-                full = {own, rows, w, s};
-            const long long times = (all + rows - 1) / rows;
-            if (!least.rows || w * times < least.warps) least = {own, rows, w * times, s * times};
+    const int last = std::min(fewest + 24, (nx + 25) / 26 + 1);
+    for (int nseg = fewest; nseg <= last; ++nseg) {
+        const int own = (nx + nseg - 1) / nseg, s = (nx + own - 1) / own;
+        for (int rows = 1, points = own + 6, faces = own + 1; points <= NT;
+             ++rows, points += own + 6, faces += own + 1) {
+            const int w = s * ((points + 31) / 32 + (faces + 31) / 32);
+            // fewer warps per row, or as many in fewer blocks
+            const long long more = (long long)w * rows_full - (long long)warps_full * rows;
+            if (!rows_full || more < 0 ||
+                (more == 0 && (long long)s * rows_full < (long long)blocks_full * rows))
+                own_full = own, rows_full = rows, warps_full = w, blocks_full = s;
+            const long long launch = (long long)w * ((all + rows - 1) / rows);
+            if (!least || launch < least) least = launch, own_least = own, rows_least = rows;
         }
     }
-    const bool fills = 3 * full.blocks * ((all + full.rows - 1) / full.rows) >= 2 * kPlaces;
-    P.own[0] = fills ? full.own : least.own, P.rows = fills ? full.rows : least.rows;
+    const long long x_blocks = (long long)blocks_full * ((all + rows_full - 1) / rows_full);
+    const bool fills = 3 * x_blocks >= 2 * kPlaces;
+    P.own[0] = fills ? own_full : own_least, P.rows = fills ? rows_full : rows_least;
     const int nxb = (nx + C - 1) / C;
     P.y0 = nxb * ny * ((nz + P.own[2] - 1) / P.own[2]);
     P.x0 = P.y0 + nxb * nz * ((ny + P.own[1] - 1) / P.own[1]);
-    P.blocks = P.x0 + (int)((all + P.rows - 1) / P.rows) * ((nx + P.own[0] - 1) / P.own[0]);
+    P.blocks = P.x0 + ((all + P.rows - 1) / P.rows) * ((nx + P.own[0] - 1) / P.own[0]);
     int t = P.rows * (P.own[0] + 6);
     for (int d = 1; d < 3; ++d) t = t > C * (P.own[d] + 6) ? t : C * (P.own[d] + 6);
     P.threads = (t + 31) / 32 * 32;
