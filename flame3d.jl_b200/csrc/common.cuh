@@ -791,13 +791,15 @@ __device__ __forceinline__ void mixture_point(const FlameThermo &th, const Flame
                                               const MixTables<NS, MT> &mt, double T, double P,
                                               double rho_raw, const double *r, double &mu,
                                               double &lam, double *Dk) {
-    const double rhoinv = fast_rcp(jmax(rho_raw, kEps));
+    // Y2X with correctly rounded quotients (fast_div), as the reference's: where a species is alone
+    // its D_k = (1 - X_k) / (Σ + eps) is a quotient of their rounding errors
+    const double rhoinv = fast_div(1.0, jmax(rho_raw, kEps));
     double X[NS];
     double yow = 0;
 #pragma unroll
     for (int n = 0; n < NS; ++n)
         X[n] = fast_div(jmax(r[n] * rhoinv, 0.0), th.mw[n]), yow += X[n];
-    const double yowinv = fast_rcp(yow);
+    const double yowinv = fast_div(1.0, yow);
 #pragma unroll
     for (int n = 0; n < NS; ++n) X[n] *= yowinv;
     if constexpr (sizeof(MT) == 8) {
